@@ -177,12 +177,19 @@ __device__ __forceinline__ void load6(const T *f, long long V, long long v, doub
   for (int c = 0; c < 6; ++c) x[c] = (double)f[c * V + v];
 }
 
-// Threads of a constitutive block, and points of one item (four per thread).
+// Threads of a constitutive block, and points of one item: four per thread, fewer (down to
+// one) where that many would leave the chip's blocks (three on each of 148 SMs) without one.
 #define CONST_THREADS 128
-#define CONST_POINTS (4 * CONST_THREADS)
+#define CONST_ROUND_ITEMS 444
 
+__host__ __device__ inline int const_chunk(long long V) {
+  for (int k = 4; k > 1; --k)
+    if (V >= (long long)k * CONST_THREADS * CONST_ROUND_ITEMS) return k * CONST_THREADS;
+  return CONST_THREADS;
+}
 __host__ __device__ inline int const_items(long long V) {
-  return (int)((V + CONST_POINTS - 1) / CONST_POINTS);
+  const int c = const_chunk(V);
+  return (int)((V + c - 1) / c);
 }
 
 // The constitutive call of one slot: strain and stress guess in, stress and tangent out,
@@ -267,7 +274,7 @@ template <typename T>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     j2_count_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ int blk_n, blk_any, blk_fail;
-  const int per = const_items(V);
+  const int chunk = const_chunk(V), per = const_items(V);
   const int n_items = list_items(list, per);
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
   const int kslot = item / per;
@@ -283,8 +290,8 @@ __global__ void __launch_bounds__(SSFFT_THREADS)
   }
   __syncthreads();
   int my_n = 0, my_any = 0, my_fail = 0;
-  const long long v1 = min(V, (long long)(local + 1) * CONST_POINTS);
-  for (long long v = (long long)local * CONST_POINTS + threadIdx.x; v < v1; v += blockDim.x) {
+  const long long v1 = min(V, (long long)(local + 1) * chunk);
+  for (long long v = (long long)local * chunk + threadIdx.x; v < v1; v += blockDim.x) {
     const PhaseParams &P = a.params[a.phase ? a.phase[v] : 0];
     if (P.kind != PHASE_J2) continue;
     double eps[6], epo[6], s[6], mean, q;
@@ -344,7 +351,7 @@ __global__ void __launch_bounds__(CONST_THREADS, 3)
 #define TS(arr, k) arr[(k) * CONST_THREADS]
   __shared__ int blk_max;
   __shared__ int blk_fail;
-  const int per = const_items(V);
+  const int chunk = const_chunk(V), per = const_items(V);
   const int n_items = list_items(list, per);
   int staged = -1;  // slot whose phase table is in shared memory
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
@@ -367,8 +374,8 @@ __global__ void __launch_bounds__(CONST_THREADS, 3)
   __syncthreads();
   int my_iters = 0;
   bool my_fail = false;
-  const long long v1 = min(V, (long long)(local + 1) * CONST_POINTS);
-  for (long long v = (long long)local * CONST_POINTS + tid; v < v1; v += CONST_THREADS) {
+  const long long v1 = min(V, (long long)(local + 1) * chunk);
+  for (long long v = (long long)local * chunk + tid; v < v1; v += CONST_THREADS) {
     const int ph = a.phase ? a.phase[v] : 0;
     const PhaseParams &P = sp[ph];
     double eps[6];

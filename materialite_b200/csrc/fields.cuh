@@ -60,14 +60,14 @@ __device__ __forceinline__ TangentRef<T> tangent_of(const SlotDev<T> &S, bool co
 template <typename T>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     strain_guess_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
-  const int per = vec_items(V);
+  const int chunk = vec_chunk(V), per = vec_items(V);
   const int n_items = list_items(list, per);
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const int k = item / per;
     const int local = item - k * per;
     const SlotDev<T> &S = tab[list.ids[k]];
-    const long long v0 = (long long)local * VEC_CHUNK;
-    const long long v1 = min(V, v0 + VEC_CHUNK);
+    const long long v0 = (long long)local * chunk;
+    const long long v1 = min(V, v0 + chunk);
     const StepVec sv = S.sv;
     const bool first = S.first_step != 0, reset = S.reset_fluct != 0;
     const double fs = S.fluct_scale;
@@ -102,15 +102,15 @@ template <typename T>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     update_strain_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   const long long n = 6 * V;
-  const int per = vec_items(n);
+  const int chunk = vec_chunk(n), per = vec_items(n);
   const int n_items = list_items(list, per);
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const int k = item / per;
     const int local = item - k * per;
     const SlotDev<T> &S = tab[list.ids[k]];
     const T *dx = S.kr[5];
-    const long long i0 = (long long)local * VEC_CHUNK;
-    const long long i1 = min(n, i0 + VEC_CHUNK);
+    const long long i0 = (long long)local * chunk;
+    const long long i1 = min(n, i0 + chunk);
     for (long long i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
       const double d = dx[i];
       S.eps[i] += d;
@@ -138,7 +138,6 @@ __device__ __forceinline__ double dev_norm6(const double *s) {
 //   out[12]    max |dev(stress - old_stress)|   out[13] max |K : dx|  (if norms_dx)
 #define NORM_VALS 14
 #define NORM_SUMS 12  // values 0..11 are sums, 12..13 maxima
-#define NORM_CHUNK (4 * SSFFT_THREADS)  // points per item
 
 // Combine one of the norm values (sum or max) in a fixed order.
 __device__ __forceinline__ double norm_combine(int k, double a, double b) {
@@ -152,13 +151,11 @@ __device__ __forceinline__ double norm_warp_reduce(int k, double v) {
   return v;
 }
 
-__host__ __device__ inline int norm_items(long long V) { return (int)((V + NORM_CHUNK - 1) / NORM_CHUNK); }
-
 template <typename T>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     newton_norms_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ double wred[NORM_VALS][SSFFT_THREADS / 32];
-  const int per = norm_items(V);
+  const int chunk = vec_chunk(V), per = vec_items(V);
   const int n_items = list_items(list, per);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
@@ -170,8 +167,8 @@ __global__ void __launch_bounds__(SSFFT_THREADS)
     double acc[NORM_VALS];
 #pragma unroll
     for (int k = 0; k < NORM_VALS; ++k) acc[k] = 0.0;
-    const long long v0 = (long long)local * NORM_CHUNK;
-    const long long v1 = min(V, v0 + NORM_CHUNK);
+    const long long v0 = (long long)local * chunk;
+    const long long v1 = min(V, v0 + chunk);
     for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
       double s[6], d[6];
 #pragma unroll
@@ -228,7 +225,7 @@ template <typename T>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     tangent_sum_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ double red[32];
-  const int per = vec_items(V);
+  const int chunk = vec_chunk(V), per = vec_items(V);
   const int n_items = list_items(list, per);
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const int kslot = item / per;
@@ -238,8 +235,8 @@ __global__ void __launch_bounds__(SSFFT_THREADS)
     double acc[21];
 #pragma unroll
     for (int k = 0; k < 21; ++k) acc[k] = 0.0;
-    const long long v0 = (long long)local * VEC_CHUNK;
-    const long long v1 = min(V, v0 + VEC_CHUNK);
+    const long long v0 = (long long)local * chunk;
+    const long long v1 = min(V, v0 + chunk);
     for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
 #pragma unroll
       for (int k = 0; k < 21; ++k) acc[k] += K.entry(v, k);
@@ -268,7 +265,7 @@ __global__ void __launch_bounds__(SSFFT_THREADS)
     commit_slip_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V,
                        int nslip_max) {
   const long long n = (long long)nslip_max * V;
-  const int per = vec_items(n);
+  const int chunk = vec_chunk(n), per = vec_items(n);
   const int n_items = list_items(list, per);
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const int k = item / per;
@@ -276,8 +273,8 @@ __global__ void __launch_bounds__(SSFFT_THREADS)
     const SlotDev<T> &S = tab[list.ids[k]];
     if (!S.any_evp) continue;
     const long long ns = (long long)S.nslip * V;
-    const long long i0 = (long long)local * VEC_CHUNK;
-    const long long i1 = min(ns, i0 + VEC_CHUNK);
+    const long long i0 = (long long)local * chunk;
+    const long long i1 = min(ns, i0 + chunk);
     for (long long i = i0 + threadIdx.x; i < i1; i += blockDim.x) S.g_old[i] = S.g_in[i];
   }
 }

@@ -430,7 +430,7 @@ static int plan_create(GridPlan &p, const ssfft_config *cfg, cudaStream_t stream
   size_t need = 0;
   need = std::max(need, (size_t)3 * items_z(g));
   need = std::max(need, (size_t)3 * CLUSTER_MAX * items_plane(g));
-  need = std::max(need, (size_t)NORM_VALS * norm_items(p.V));
+  need = std::max(need, (size_t)NORM_VALS * vec_items(p.V));
   need = std::max(need, (size_t)21 * vec_items(p.V));
   need = std::max(need, (size_t)vec_items(6 * p.V));
   if (items_z(g) > MAX_ITEMS_PER_SLOT || vec_items(6 * p.V) > MAX_ITEMS_PER_SLOT ||
@@ -1043,7 +1043,7 @@ template <typename T> static int launch_update_strain(const LaunchCtx &c, const 
 
 template <typename T> static int launch_norms(const LaunchCtx &c, const SlotDev<T> *tab) {
   auto k = newton_norms_kernel<T>;
-  const long long it = (long long)c.cap * norm_items(c.p->V);
+  const long long it = (long long)c.cap * vec_items(c.p->V);
   k<<<persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0, c.stream>>>(tab, c.list, c.p->V);
   if (c.launches) *c.launches += 1;
   CK(cudaGetLastError());

@@ -440,7 +440,7 @@ extern "C" int ssfft_estimate_bytes(const ssfft_config *cfg, int any_evp, int n_
   // strain and stress fields double in both precisions, the rest in the solve precision
   size_t b = 6 * 6 * V * 8 + 8 * 6 * V * rs + 6 * S * 16 + 3 * V * 4;
   if (any_evp) b += 2 * 21 * V * rs + (5 * (size_t)n_slip + 12 + 2) * V * 8;
-  b += (size_t)21 * ((V + VEC_CHUNK - 1) / VEC_CHUNK + 1) * 8 + 3 * 3 * (size_t)cfg->n[0] * 8;
+  b += (size_t)21 * (vec_items((long long)V) + 1) * 8 + 3 * 3 * (size_t)cfg->n[0] * 8;
   b += (size_t)1 << 20;  // tables, scalars, orientation table
   *bytes = b;
   return 0;
