@@ -13,7 +13,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.dirname(HERE)
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3",
-              "--threads", "0", "--split-compile", "0",
+              "--threads", "0",
               "-std=c++17", "-shared", "-Xcompiler", "-fPIC,-O2"]
 
 

@@ -324,6 +324,7 @@ struct Group {
   std::vector<SlotBufs> slots;
   std::vector<bool> allocated;
   void *dtab = nullptr;        // SlotDev<T>[B]
+  MinresState *dst = nullptr;  // [B]
   GroupCtl *dctl = nullptr;
   GroupCtl *hctl = nullptr;    // pinned mirror
   int *dids = nullptr;         // [GL_COUNT][B]
@@ -350,10 +351,11 @@ struct Group {
       if (allocated[s]) slot_free(slots[s]);
     slots.clear();
     allocated.clear();
-    void *ptrs[] = {dtab, dctl, dids, dcounts, dloop, stage};
+    void *ptrs[] = {dtab, dst, dctl, dids, dcounts, dloop, stage};
     for (void *p : ptrs)
       if (p) cudaFree(p);
     dtab = nullptr;
+    dst = nullptr;
     dctl = nullptr;
     dids = dcounts = nullptr;
     dloop = nullptr;
@@ -387,6 +389,7 @@ struct Group {
     allocated.assign(B, false);
     ALLOC(dtab, desc_bytes() * B);
     CK(cudaMemsetAsync(dtab, 0, desc_bytes() * B, stream));
+    ALLOC(dst, sizeof(MinresState) * B);
     ALLOC(dctl, sizeof(GroupCtl) * B);
     CK(cudaMemsetAsync(dctl, 0, sizeof(GroupCtl) * B, stream));
     ALLOC(dids, sizeof(int) * GL_COUNT * B);
@@ -410,6 +413,7 @@ struct Group {
 
   SlotList list(int l) const {
     SlotList L;
+    L.st = dst;
     L.ids = dids + l * B;
     L.count = dcounts + l;
     return L;
@@ -463,8 +467,9 @@ struct Group {
 
   template <typename T> int issue_chunk(cudaStream_t s) {
     SlotDev<T> *tab = (SlotDev<T> *)dtab;
+    // the first kernel may follow a conditional node, which programmatic launches cannot
     for (int i = 0; i < GROUP_KRYLOV_CHUNK; ++i)
-      CKR(launch_krylov_iteration<T>(lctx(GL_KRY, s), tab, voxel));
+      CKR(launch_krylov_iteration<T>(lctx(GL_KRY, s), tab, voxel, nullptr, i > 0));
     return 0;
   }
 
@@ -582,7 +587,7 @@ struct Group {
     CK(cudaSetDevice(device));
     SlotBufs &b = slots[s];
     if (!allocated[s]) {
-      CKR(slot_alloc(b, plan, stream));
+      CKR(slot_alloc(b, plan, stream, dst + s));
       allocated[s] = true;
     }
     ssfft_config cfg = j.req.config;

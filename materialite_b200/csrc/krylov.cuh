@@ -142,14 +142,21 @@ __global__ void __launch_bounds__(SSFFT_THREADS)
   __shared__ double red[32];
   __shared__ __align__(16) unsigned char sdesc[sizeof(SlotDev<T>)];
   const int chunk = vec_chunk(V), per = vec_items(V);
+  pdl_begin();
+  pdl_wait();
+  const int slot0 = list.ids[blockIdx.x / per];  // read beside the count: a grid has no more blocks than the list can fill
   const int n_items = list_items(list, per);
   int staged = -1;
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const int k = item / per;
     const int local = item - k * per;
-    const SlotDev<T> &S = stage_slot<T>(tab, list.ids[k], sdesc, staged);
-    if (slot_done(S.st)) continue;
-    const KrylovIn<T, T> u = krylov_in<T, T>(S);
+    const int slot = item == (int)blockIdx.x ? slot0 : list.ids[k];
+    const MinresState *st = list.st + slot;
+    const bool done = slot_done(st);
+    KrylovIn<T, T> u = krylov_in<T, T>(st);
+    const SlotDev<T> &S = stage_slot<T>(tab, slot, sdesc, staged);
+    if (done) continue;
+    u.r = kroles<T>(S, u.itn);
     const long long v0 = (long long)local * chunk;
     const long long v1 = min(V, v0 + chunk);
     T *tau_out = u.r.Y;
@@ -174,15 +181,22 @@ __global__ void __launch_bounds__(SSFFT_THREADS)
   __shared__ double red[32];
   __shared__ __align__(16) unsigned char sdesc[sizeof(SlotDev<T>)];
   const int chunk = vec_chunk(V), per = vec_items(V);
+  pdl_begin();
+  pdl_wait();
+  const int slot0 = list.ids[blockIdx.x / per];  // read beside the count: a grid has no more blocks than the list can fill
   const int n_items = list_items(list, per);
   int staged = -1;
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const int k = item / per;
     const int local = item - k * per;
-    const SlotDev<T> &S = stage_slot<T>(tab, list.ids[k], sdesc, staged);
-    if (slot_done(S.st)) continue;
-    const KRoles<T> kr = kroles<T>(S, S.st->itn);
-    const T c1 = (T)S.st->c_r1;
+    const int slot = item == (int)blockIdx.x ? slot0 : list.ids[k];
+    const MinresState *st = list.st + slot;
+    const bool done = slot_done(st);
+    const long long itn = st->itn;
+    const T c1 = (T)st->c_r1;
+    const SlotDev<T> &S = stage_slot<T>(tab, slot, sdesc, staged);
+    if (done) continue;
+    const KRoles<T> kr = kroles<T>(S, itn);
     const long long v0 = (long long)local * chunk;
     const long long v1 = min(V, v0 + chunk);
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;

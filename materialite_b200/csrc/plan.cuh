@@ -18,6 +18,7 @@
 #include "../../include/ssfft.h"
 #include "common.cuh"
 #include "constitutive.cuh"
+#include "dif.cuh"
 #include "fft.cuh"
 #include "fields.cuh"
 #include "krylov.cuh"
@@ -149,6 +150,24 @@ static int launch_clustered(void (*f)(P...), int C, int threads, size_t smem, lo
   return 0;
 }
 
+// Launch of a kernel that calls pdl_wait(): with `pdl`, it may start while the kernel before it
+// in the stream still runs.
+template <typename... P, typename... A>
+static void launch_pdl(bool pdl, void (*f)(P...), int grid, int threads, size_t smem,
+                       cudaStream_t stream, A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, f, std::forward<A>(args)...);
+}
+
 // ---------------------------------------------------------------------------------------
 // grid plan
 // ---------------------------------------------------------------------------------------
@@ -169,6 +188,8 @@ struct GridPlan {
   void *tw[2][3], *tn[2][3];  // [0]: float, [1]: double tables per axis
   Grid<float> gf;
   Grid<double> gd;
+  DifPlane dplane[2][2];      // register-tiled passes: [0] float, [1] double; forward, inverse
+  DifXPlan dx[2];
   size_t partial_doubles;     // reduction partials per slot
 };
 
@@ -328,6 +349,129 @@ template <typename T> static int plane_threads(const GridPlan &p) {
   return smem_plane_bytes<T>(p.ny, p.nz) > 113 * 1024 ? 1024 : 512;
 }
 
+// ---------------------------------------------------------------------------------------
+// plans of the register-tiled passes (dif.cuh)
+// ---------------------------------------------------------------------------------------
+// Factor n into two or three stages with the first radix in `first`, the middle one at most
+// 8 and the last one in `last` (bit r: radix r).  Fewest stages, then the smallest widest
+// radix, then the larger first one.
+#define DIF_RADICES 0x117feu     // 1 .. 10, 12, 16
+#define DIF_RADICES_PAIR 0x1feu  // 1 .. 8: stages that hold two lines a thread
+static bool dif_axis(int n, unsigned first, unsigned last, DifAxis &A) {
+  memset(&A, 0, sizeof(A));
+  int best = 1 << 30;
+  auto ok = [](unsigned set, int r) { return r <= 16 && ((set >> r) & 1u); };
+  auto take = [&](int ns, int r0, int r1, int r2) {
+    const int widest = std::max(r0, std::max(r1, r2));
+    const int cost = ns * 1000 + 4 * widest - (r0 >= r1 ? 1 : 0);
+    if (cost >= best) return;
+    best = cost;
+    A.ns = ns;
+    A.r0 = r0;
+    A.r1 = r1;
+    A.r2 = r2;
+  };
+  for (int r0 = 1; r0 <= 16; ++r0) {
+    if (!ok(first, r0) || n % r0) continue;
+    const int m = n / r0;
+    if (ok(last, m)) take(2, r0, m, 1);
+    for (int r1 = 2; r1 <= 8; ++r1)
+      if (m % r1 == 0 && ok(last, m / r1)) take(3, r0, r1, m / r1);
+  }
+  if (A.ns == 0) return false;
+  A.n = n;
+  A.m = n / A.r0;
+  const int rl = A.ns == 2 ? A.r1 : A.r2;
+  A.fd_m = make_fastdiv((uint32_t)A.m);
+  A.fd_r0 = make_fastdiv((uint32_t)A.r0);
+  A.fd_nb = make_fastdiv((uint32_t)(n / rl));
+  A.fd_nb1 = make_fastdiv((uint32_t)(A.r0 * A.r2));
+  return true;
+}
+
+#define DIF_SMEM_LIMIT (224 * 1024)
+// Smaller planes stay on the Stockham passes, whose kernels start faster: a 16^3 projection
+// takes 36 us there and 40 us in the register-tiled passes; 30 x 28 x 27 takes 52 and 41.
+#define DIF_MIN_PLANE 512
+
+// Plan of the forward (inv = false) or inverse plane pass in one block's buffer (ok = 0 where
+// an axis has no plan or the plane is too large).
+template <typename T> static DifPlane dif_plane(int ny, int nz, int hs, bool inv) {
+  DifPlane P;
+  memset(&P, 0, sizeof(P));
+  if (!dif_axis(nz, inv ? DIF_RADICES_PAIR : DIF_RADICES, inv ? DIF_RADICES : DIF_RADICES_PAIR, P.z) ||
+      !dif_axis(ny, DIF_RADICES, DIF_RADICES, P.y))
+    return P;
+  P.z.a = P.z.r0 | 1;  // odd
+  P.z.b = 1;
+  P.ls = P.z.m * P.z.a;
+  // column (1, 0): the padding slot of n' = 0, or one more slot a row where there is none
+  P.xslot = (P.z.r0 & 1) ? P.ls++ : P.z.r0;
+  const int nb = nz / (P.z.ns == 2 ? P.z.r1 : P.z.r2);
+  P.z.fd_un = make_fastdiv((uint32_t)((inv ? P.z.m : nb) / 2 + 1));
+  P.elems = ny * P.ls;
+  P.y.a = P.ls;
+  P.y.b = P.y.m * P.ls;
+  P.y.fd_un = make_fastdiv((uint32_t)P.ls);  // slots to rows
+  const size_t bytes = DifTables<T, false>::bytes(P, ny, nz, hs);
+  P.ok = bytes <= DIF_SMEM_LIMIT && P.ls < 65536 ? 1 : 0;
+  // about one radix-8 butterfly a thread and stage
+  // (up to 1024 in float where one block fills an SM: 32 warps instead of 16)
+  const int most = sizeof(T) == 4 && bytes > 112 * 1024 ? 1024 : 512;
+  P.threads = std::max(64, std::min(most, (ny * nz / 8 + 63) / 64 * 64));
+  return P;
+}
+
+// x pass: tiles take 64-byte runs of a spectrum row, halved (down to a 32-byte sector) while
+// the grid then has fewer than four tiles an SM and while a tile exceeds 40 KB (five blocks an
+// SM).
+template <typename T> static DifXPlan dif_xplan(int nx, int ny, int hs) {
+  DifXPlan P;
+  memset(&P, 0, sizeof(P));
+  DifAxis &X = P.x;
+  if (!dif_axis(nx, DIF_RADICES, DIF_RADICES, X)) return P;
+  const int sector = 32 / (int)sizeof(cplx<T>);
+  const int w = 128 / (int)sizeof(cplx<T>);
+  P.kx = 64 / (int)sizeof(cplx<T>);
+  auto layout = [&]() {
+    const int run = X.r0 * P.kx;
+    X.a = run + ((P.kx - run) % w + w) % w;
+    X.b = P.kx;
+    P.cs = X.m * X.a;
+    P.elems = 6 * P.cs;
+    P.nkx = (hs + P.kx - 1) / P.kx;
+    return ((size_t)P.elems + nx) * sizeof(cplx<T>);
+  };
+  while (P.kx > sector && ((long long)((hs + P.kx - 1) / P.kx) * ny < 4 * 148 || P.kx >= 2 * hs)) P.kx /= 2;
+  while (layout() > 40 * 1024 && P.kx > sector) P.kx /= 2;
+  while (layout() > SMEM_LIMIT && P.kx > 1) P.kx /= 2;
+  if (layout() > SMEM_LIMIT) return P;
+  while ((1 << P.lkx) < P.kx) ++P.lkx;
+  P.fd_mid = make_fastdiv((uint32_t)(X.r0 * P.kx));
+  P.fd_r2 = make_fastdiv((uint32_t)X.r2);
+  P.fd_items = make_fastdiv((uint32_t)(P.nkx * ny));
+  P.fd_nkx = make_fastdiv((uint32_t)P.nkx);
+  P.ok = 1;
+  return P;
+}
+
+// x pass of a launch: the register-tiled one where nx has a plan for it (unless a tile shape
+// of the Stockham pass is asked for), else the Stockham one.
+template <typename T, typename TF, bool KRY>
+static void launch_x(const GridPlan &p, const Grid<T> &g, long long cap, cudaStream_t stream,
+                     const SlotDev<TF> *tab, SlotList list) {
+  const DifXPlan &P = p.dx[sizeof(T) == 8 ? 1 : 0];
+  if (!P.ok) {
+    launch_xpass<T, TF, KRY>(g, smem_x_bytes<T>(g.kx, p.nx), cap * items_x(g), p.dev, stream, tab, list);
+    return;
+  }
+  auto k = difx_kernel<T>;
+  const size_t sm = ((size_t)P.elems + p.nx) * sizeof(cplx<T>);
+  const int grid = persistent_grid(k, DIFX_THREADS, sm, cap * P.nkx * p.ny, p.dev);
+  launch_pdl(true, k, grid, DIFX_THREADS, sm, stream, g, P, reinterpret_cast<const SlotDev<T> *>(tab),
+             list, KRY ? 1 : 0);
+}
+
 static int validate_config(const ssfft_config *cfg) {
   if (!cfg) return ssfft_internal_fail(SSFFT_E_INVALID, "null config");
   for (int d = 0; d < 3; ++d)
@@ -382,7 +526,7 @@ static void plan_free(GridPlan &p) {
     }
 }
 
-template <typename T, typename TF> static int set_kernel_attrs(size_t smax);
+template <typename T, typename TF> static int set_kernel_attrs(const GridPlan &p, size_t smax);
 
 static int plan_create(GridPlan &p, const ssfft_config *cfg, cudaStream_t stream) {
   memset(&p, 0, sizeof(p));
@@ -425,6 +569,16 @@ static int plan_create(GridPlan &p, const ssfft_config *cfg, cudaStream_t stream
     }
   fill_grid<double>(p);
   if (!p.fp64) fill_grid<float>(p);
+  if (p.use_plane && env_int("SSFFT_CLUSTER") <= 0 && p.ny * p.nz >= DIF_MIN_PLANE) {
+    for (int d = 0; d < 2; ++d) {
+      p.dplane[0][d] = dif_plane<float>(p.ny, p.nz, p.gd.hs, d == 1);
+      p.dplane[1][d] = dif_plane<double>(p.ny, p.nz, p.gd.hs, d == 1);
+    }
+  }
+  if (p.ny * p.nz >= DIF_MIN_PLANE && env_int("SSFFT_XPASS_KX") <= 0 && env_int("SSFFT_XPASS_THREADS") <= 0) {
+    p.dx[0] = dif_xplan<float>(p.nx, p.ny, p.gd.hs);
+    p.dx[1] = dif_xplan<double>(p.nx, p.ny, p.gd.hs);
+  }
   // items of one slot per reduction, times the values each stores
   const Grid<double> &g = p.gd;
   size_t need = 0;
@@ -437,9 +591,12 @@ static int plan_create(GridPlan &p, const ssfft_config *cfg, cudaStream_t stream
       items_y(g) > (1 << 30) / 2)
     return ssfft_internal_fail(SSFFT_E_UNSUPPORTED, "grid too large for the reduction partials");
   p.partial_doubles = need;
-  CKR((set_kernel_attrs<double, double>(SMEM_LIMIT)));
-  CKR((set_kernel_attrs<float, float>(SMEM_LIMIT)));
-  CKR((set_kernel_attrs<double, float>(SMEM_LIMIT)));
+  if (p.fp64) {
+    CKR((set_kernel_attrs<double, double>(p, SMEM_LIMIT)));
+  } else {
+    CKR((set_kernel_attrs<float, float>(p, SMEM_LIMIT)));
+    CKR((set_kernel_attrs<double, float>(p, SMEM_LIMIT)));
+  }
   return 0;
 }
 
@@ -479,9 +636,38 @@ template <typename T, typename TF, int PT> static int cluster_attrs(int m) {
   return 0;
 }
 
-// Opt every shared-memory-hungry kernel instantiation into up to `smax` bytes.
-template <typename T, typename TF> static int set_kernel_attrs(size_t smax) {
+// The plane-pass instantiations of transforms in T with planes stored in TF.
+template <typename T, typename TF> static int dif_plane_attrs() {
+  const int m = DIF_SMEM_LIMIT;
+  CKR((smem_attr(dif_zyfwd_kernel<T, TF, DIF_PLANES>, m)));
+  if constexpr (sizeof(T) == sizeof(TF)) CKR((smem_attr(dif_yzinv_kernel<T, TF, DIF_PLANES>, m)));
+  if constexpr (sizeof(T) == 8) {
+    CKR((smem_attr(dif_zyfwd_kernel<double, double, DIF_RESIDUAL>, m)));
+    CKR((smem_attr(dif_yzinv_kernel<T, TF, DIF_RESIDUAL>, m)));
+    if constexpr (sizeof(TF) == 4) CKR((smem_attr(dif_yzinv_kernel<T, TF, DIF_REPROJECT>, m)));
+  }
+  return 0;
+}
+
+// Opt the shared-memory-hungry kernels of the plan's paths into up to `smax` bytes (the others
+// are not touched: the first touch of a kernel loads its code).
+template <typename T, typename TF> static int set_kernel_attrs(const GridPlan &p, size_t smax) {
   const int m = (int)smax;
+  const int k = sizeof(T) == 8 ? 1 : 0;
+  if constexpr (sizeof(T) == sizeof(TF)) CKR(smem_attr(constitutive_kernel<T>, (int)constitutive_smem_bytes()));
+  if (p.dx[k].ok) {
+    CKR(smem_attr(difx_kernel<T>, m));
+  } else {
+    CKR((smem_attr(xpass_kernel<T, TF, false>, m)));
+    CKR((smem_attr(xpass_kernel<T, TF, true>, m)));
+    if constexpr (sizeof(T) == 4) {
+      CKR((smem_attr(xpass_kernel<T, TF, false, 192>, m)));
+      CKR((smem_attr(xpass_kernel<T, TF, true, 192>, m)));
+      CKR((smem_attr(xpass_kernel<T, TF, false, 384>, m)));
+      CKR((smem_attr(xpass_kernel<T, TF, true, 384>, m)));
+    }
+  }
+  if (p.dplane[k][0].ok && p.dplane[k][1].ok) return dif_plane_attrs<T, TF>();
   CKR(smem_attr(zfwd_kernel<T, TF, PRO_INPUT>, m));
   CKR(smem_attr(zfwd_kernel<T, TF, PRO_RESIDUAL>, m));
   CKR(smem_attr(zfwd_kernel<T, TF, PRO_REPROJECT>, m));
@@ -489,14 +675,6 @@ template <typename T, typename TF> static int set_kernel_attrs(size_t smax) {
   CKR((smem_attr(ypass_kernel<T, TF, true, false>, m)));
   CKR((smem_attr(ypass_kernel<T, TF, false, true>, m)));
   CKR((smem_attr(ypass_kernel<T, TF, true, true>, m)));
-  CKR((smem_attr(xpass_kernel<T, TF, false>, m)));
-  CKR((smem_attr(xpass_kernel<T, TF, true>, m)));
-  if constexpr (sizeof(T) == 4) {
-    CKR((smem_attr(xpass_kernel<T, TF, false, 192>, m)));
-    CKR((smem_attr(xpass_kernel<T, TF, true, 192>, m)));
-    CKR((smem_attr(xpass_kernel<T, TF, false, 384>, m)));
-    CKR((smem_attr(xpass_kernel<T, TF, true, 384>, m)));
-  }
   CKR(smem_attr(zinv_kernel<T, TF, EPI_STORE>, m));
   CKR(smem_attr(zinv_kernel<T, TF, EPI_RESIDUAL>, m));
   CKR(smem_attr(zinv_kernel<T, TF, EPI_REPROJECT>, m));
@@ -506,7 +684,6 @@ template <typename T, typename TF> static int set_kernel_attrs(size_t smax) {
   CKR((cluster_attrs<T, TF, 512>(m)));
   CKR((cluster_attrs<T, TF, 1024>(m)));
   if (sizeof(T) == sizeof(TF)) {
-    CKR(smem_attr(constitutive_kernel<T>, (int)constitutive_smem_bytes()));
     CKR(smem_attr(zfwd_kernel<T, T, PRO_TAU>, m));
     CKR(smem_attr(zinv_kernel<T, T, EPI_PTAU>, m));
   }
@@ -528,6 +705,7 @@ struct SlotBufs {
   unsigned int *tickets;
   double *results;
   MinresState *st;
+  bool st_shared;              // st is the caller's
   int *citers;
   // microstructure (capacities grow on rebinding)
   PhaseParams hparams[SSFFT_MAX_PHASES];
@@ -560,7 +738,9 @@ static size_t field_bytes_of(const SlotBufs &b, int i) {
   return i < 6 ? (size_t)6 * (size_t)b.V * sizeof(double) : field_bytes(b, 6);
 }
 
-static int slot_alloc(SlotBufs &b, const GridPlan &p, cudaStream_t stream) {
+// st: the slot's MINRES state where the caller owns it (a group keeps its slots' states in
+// one array), else one is allocated.
+static int slot_alloc(SlotBufs &b, const GridPlan &p, cudaStream_t stream, MinresState *st = nullptr) {
   memset((void *)&b, 0, sizeof(b));
   b.fp64 = p.fp64;
   b.rs = p.fp64 ? 8 : 4;
@@ -575,7 +755,12 @@ static int slot_alloc(SlotBufs &b, const GridPlan &p, cudaStream_t stream) {
   CK(cudaMemsetAsync(b.tickets, 0, 16 * sizeof(unsigned int), stream));
   ALLOC(b.results, 64 * sizeof(double));
   CK(cudaMemsetAsync(b.results, 0, 64 * sizeof(double), stream));
-  ALLOC(b.st, sizeof(MinresState));
+  if (st) {
+    b.st = st;
+    b.st_shared = true;
+  } else {
+    ALLOC(b.st, sizeof(MinresState));
+  }
   CK(cudaMemsetAsync(b.st, 0, sizeof(MinresState), stream));
   ALLOC(b.citers, 4 * sizeof(int));
   CK(cudaMemsetAsync(b.citers, 0, 4 * sizeof(int), stream));
@@ -584,7 +769,7 @@ static int slot_alloc(SlotBufs &b, const GridPlan &p, cudaStream_t stream) {
 }
 
 static void slot_free(SlotBufs &b) {
-  void *ptrs[] = {b.spec, b.partials, b.tickets, b.results, b.st, b.citers, b.dparams,
+  void *ptrs[] = {b.spec, b.partials, b.tickets, b.results, b.st_shared ? nullptr : b.st, b.citers, b.dparams,
                   b.orient, b.phase, b.gid, b.rm_tab, b.ktab, b.kvox_buf[0], b.kvox_buf[1],
                   b.slip_buf[0], b.slip_buf[1], b.slip_buf[2], b.slip_buf[3], b.slip_buf[4],
                   b.ep_buf[0], b.ep_buf[1], b.Gam_buf[0], b.Gam_buf[1]};
@@ -881,6 +1066,39 @@ struct LaunchCtx {
   long long *launches;
 };
 
+// The register-tiled plane passes of one projection around the x pass.
+template <typename T, typename TF, int PRO, int EPI, typename REC>
+static void launch_dif_planes(const LaunchCtx &c, const SlotDev<TF> *tab, const ExtIO<TF> &io,
+                              const DifPlane *PP, const REC &rec) {
+  const DifPlane &P = PP[0], &Q = PP[1];
+  constexpr bool KRY = PRO == PRO_TAU;
+  const GridPlan &p = *c.p;
+  const Grid<T> &g = grid_of<T>(p);
+  const size_t sp = DifTables<T, false>::bytes(P, p.ny, p.nz, g.hs);
+  const size_t sq = DifTables<T, true>::bytes(Q, p.ny, p.nz, g.hs);
+  const long long it = (long long)c.cap * items_plane(g);
+  const int pt = P.threads;
+  if constexpr (PRO == PRO_RESIDUAL) {
+    // the residual reads the stress alone, which is double for either storage type
+    auto kf = dif_zyfwd_kernel<double, double, DIF_RESIDUAL>;
+    launch_pdl(false, kf, persistent_grid(kf, pt, sp, it, p.dev), pt, sp, c.stream, g, P,
+               reinterpret_cast<const SlotDev<double> *>(tab), c.list, ExtIO<double>{}, (int)PRO);
+  } else {
+    auto kf = dif_zyfwd_kernel<T, TF, DIF_PLANES>;
+    launch_pdl(KRY, kf, persistent_grid(kf, pt, sp, it, p.dev), pt, sp, c.stream, g, P, tab, c.list,
+               io, (int)PRO);
+  }
+  rec(1);
+  rec(2);
+  launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list);
+  rec(3);
+  rec(4);
+  constexpr int KIND = EPI == EPI_RESIDUAL ? DIF_RESIDUAL : (EPI == EPI_REPROJECT ? DIF_REPROJECT : DIF_PLANES);
+  auto ki = dif_yzinv_kernel<T, TF, KIND>;
+  launch_pdl(true, ki, persistent_grid(ki, pt, sq, it, p.dev), pt, sq, c.stream, g, Q, tab, c.list, io,
+             (int)EPI);
+}
+
 // The passes of one projection.  ev (optional, 6 events) is recorded before the first pass
 // and after each of the five pass slots z-fwd, y-fwd, x, y-inv, z-inv; with the
 // plane-fused passes the y slots are empty (zero time).
@@ -895,10 +1113,14 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
   auto rec = [&](int k) {
     if (ev) cudaEventRecord(ev[k], c.stream);
   };
-  const size_t sx = smem_x_bytes<T>(g.kx, p.nx);
   const int dev = p.dev;
+  const DifPlane *dp = p.dplane[sizeof(T) == 8 ? 1 : 0];
   rec(0);
-  if (const int C = cluster_size<T>(p)) {
+  if (dp[0].ok && dp[1].ok) {
+    launch_dif_planes<T, TF, PRO, EPI>(c, tab, io, dp, rec);
+    rec(5);
+    if (c.launches) *c.launches += 3;
+  } else if (const int C = cluster_size<T>(p)) {
     const ClusterGeo q = cluster_geo<T>(p, C);
     const size_t sp = smem_cplane_bytes<T>(p.ny, p.nz, g.hs, C);
     const long long it = (long long)c.cap * items_plane(g);
@@ -911,7 +1133,7 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
       CKR(launch_clustered(zyfwd_cl_kernel<T, TF, PRO, 512>, C, 512, sp, it, dev, c.stream, g, q, tab, c.list, io));
     rec(1);
     rec(2);
-    launch_xpass<T, TF, KRY>(g, sx, (long long)c.cap * items_x(g), dev, c.stream, tab, c.list);
+    launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list);
     rec(3);
     rec(4);
     if (pt == 1024)
@@ -934,7 +1156,7 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
     }
     rec(1);
     rec(2);
-    launch_xpass<T, TF, KRY>(g, sx, (long long)c.cap * items_x(g), dev, c.stream, tab, c.list);
+    launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list);
     rec(3);
     rec(4);
     if (plane_threads<T>(p) == 1024) {
@@ -957,7 +1179,7 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
     auto ky = ypass_kernel<T, TF, false, KRY>;
     ky<<<persistent_grid(ky, SSFFT_THREADS, sy, ity, dev), SSFFT_THREADS, sy, c.stream>>>(g, tab, c.list);
     rec(2);
-    launch_xpass<T, TF, KRY>(g, sx, (long long)c.cap * items_x(g), dev, c.stream, tab, c.list);
+    launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list);
     rec(3);
     auto kyi = ypass_kernel<T, TF, true, KRY>;
     kyi<<<persistent_grid(kyi, SSFFT_THREADS, sy, ity, dev), SSFFT_THREADS, sy, c.stream>>>(g, tab, c.list);
@@ -978,21 +1200,24 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
 // epilogue kernel follows ev[5]).
 template <typename T>
 static int launch_krylov_iteration(const LaunchCtx &c, const SlotDev<T> *tab, bool voxel,
-                                   cudaEvent_t *ev = nullptr) {
+                                   cudaEvent_t *ev = nullptr, bool pdl_first = false) {
   if (ev) cudaEventRecord(ev[7], c.stream);
   const long long it = (long long)c.cap * vec_items(c.p->V);
   if (voxel) {
     auto k = krylov_update_kernel<T, PRO_TANGENT_VOXEL>;
-    k<<<persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0, c.stream>>>(tab, c.list, c.p->V);
+    launch_pdl(pdl_first, k, persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0,
+               c.stream, tab, c.list, c.p->V);
   } else {
     auto k = krylov_update_kernel<T, PRO_TANGENT_TABLE>;
-    k<<<persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0, c.stream>>>(tab, c.list, c.p->V);
+    launch_pdl(pdl_first, k, persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0,
+               c.stream, tab, c.list, c.p->V);
   }
   if (c.launches) *c.launches += 1;
   CK(cudaGetLastError());
   CKR((launch_projector<T, T, PRO_TAU, EPI_PTAU>(c, tab, {}, ev)));
   auto ke = krylov_epilogue_kernel<T>;
-  ke<<<persistent_grid(ke, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0, c.stream>>>(tab, c.list, c.p->V);
+  launch_pdl(true, ke, persistent_grid(ke, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0, c.stream,
+             tab, c.list, c.p->V);
   if (c.launches) *c.launches += 1;
   CK(cudaGetLastError());
   return 0;
@@ -1010,7 +1235,10 @@ template <typename T> static int launch_residual(const LaunchCtx &c, const SlotD
 // then strain += x and fluctuation += x.  Float Krylov iterates pick up round-off in the
 // null space of Gamma-hat K, which the equilibrium test cannot see; this removes it.
 template <typename T> static int launch_reproject_update(const LaunchCtx &c, const SlotDev<T> *tab) {
-  return launch_projector<double, T, PRO_REPROJECT, EPI_REPROJECT>(c, tab);
+  if constexpr (sizeof(T) == 4)
+    return launch_projector<double, T, PRO_REPROJECT, EPI_REPROJECT>(c, tab);
+  else
+    return ssfft_internal_fail(SSFFT_E_INVALID, "double solves are not re-projected");
 }
 
 template <typename T>

@@ -229,19 +229,19 @@ static __device__ __noinline__ void minres_after_matvec(MinresState *st, double 
 }
 
 // Scalars of the update pending from the previous MINRES iteration (all iterations after
-// the first: itn >= 1), and the vector roles of this iteration.
+// the first: itn >= 1); the vector roles r follow from itn and the slot's descriptor.
 template <typename T, typename TF> struct KrylovIn {
   bool on;
+  long long itn;
   T s, coef, sp, oe, de, dn, ph;
   KRoles<TF> r;
 };
 
 template <typename T, typename TF>
-__device__ __forceinline__ KrylovIn<T, TF> krylov_in(const SlotDev<TF> &S) {
-  const MinresState *st = S.st;
+__device__ __forceinline__ KrylovIn<T, TF> krylov_in(const MinresState *st) {
   KrylovIn<T, TF> u;
-  const long long itn = st->itn;
-  u.on = itn >= 1;
+  u.itn = st->itn;
+  u.on = u.itn >= 1;
   u.s = (T)st->s;
   u.coef = (T)st->coef;
   u.sp = (T)st->s_prev;
@@ -249,7 +249,6 @@ __device__ __forceinline__ KrylovIn<T, TF> krylov_in(const SlotDev<TF> &S) {
   u.de = (T)st->delta;
   u.dn = (T)st->denom;
   u.ph = (T)st->phi;
-  u.r = kroles<TF>(S, itn);
   return u;
 }
 

@@ -75,11 +75,21 @@ template <typename T> struct SlotDev {
 };
 
 // The slots a launch works on: ids[0 .. *count).  Both live in device memory, so a kernel
-// captured in a CUDA graph sees the list of the moment it runs.
+// captured in a CUDA graph sees the list of the moment it runs.  st holds every slot's MINRES
+// state by slot id (what the slots' descriptors point to): a kernel reads it beside the
+// descriptor instead of after it.
 struct SlotList {
   const int *ids;
   const int *count;
+  const MinresState *st;
 };
+
+// Programmatic dependent launch: the kernels of a Krylov iteration let the next one start as
+// soon as they run, so that its launch, block start-up and table loads overlap their own work,
+// and each waits here, before its first access to anything another kernel touches, until the
+// kernels before it have finished.  Without the launch attribute both are no-ops.
+__device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Krylov vector roles at iteration itn (itn matrix-vector products done): P holds u_{j-1},
 // Q receives u_j, W the new search direction, W1 and W2 the previous two, X the iterate,

@@ -77,6 +77,7 @@ static LaunchCtx ctx(ssfft_handle *h) {
   c.p = &h->plan;
   c.list.ids = h->dlist;
   c.list.count = h->dlist + 1;
+  c.list.st = h->sb.st;
   c.cap = 1;
   c.stream = h->stream;
   c.launches = &h->launches;
@@ -129,7 +130,8 @@ template <typename T> static int run_minres(ssfft_handle *h, long long *iters) {
   // One chunk of KRYLOV_CHUNK iterations; kernels return at once when the slot's MINRES
   // state says done, and the vector roles follow the state's iteration count.
   auto chunk = [&]() -> int {
-    for (int i = 0; i < KRYLOV_CHUNK; ++i) CKR(launch_krylov_iteration<T>(c, tab, voxel));
+    for (int i = 0; i < KRYLOV_CHUNK; ++i)
+      CKR(launch_krylov_iteration<T>(c, tab, voxel, nullptr, i > 0));
     return 0;
   };
   if (h->use_device_loop) {
