@@ -291,17 +291,17 @@ static_assert(sizeof(SlotDev<float>) == sizeof(SlotDev<double>) &&
                   offsetof(SlotDev<float>, mask) == offsetof(SlotDev<double>, mask),
               "slot descriptors must have one layout");
 
-// Middle stage of the x lines (three-stage axes): butterflies (c, n'', q_0, column).
-template <typename T, bool INV>
+// Middle stage of NC components' lines (three-stage axes): butterflies (c, n'', q_0, column).
+template <typename T, bool INV, int NC = 6>
 __device__ __forceinline__ void difx_middle(SPtr<T> buf, const DifXPlan &P, SPtr<T> tw) {
   const DifAxis &X = P.x;
   const int inner = X.r0 << P.lkx;            // contiguous (q_0, column)
-  const int total = 6 * X.r2 * inner;
+  const int total = NC * X.r2 * inner;
   DIF_RADIX8(X.r1,
 _Pragma("unroll 1")
     for (int t = threadIdx.x; t < total; t += blockDim.x) {
       const int g = udiv(t, P.fd_mid), in = t - g * inner;
-      const int c = udiv(g, P.fd_r2), n2 = g - c * X.r2;
+      const int c = NC == 1 ? 0 : udiv(g, P.fd_r2), n2 = g - c * X.r2;
       const SPtr<T> b = buf + c * P.cs + n2 * X.a + in;
       const int step = X.r2 * X.a;
       cplx<T> v[R];
@@ -443,6 +443,120 @@ _Pragma("unroll")
         }
       }
     )
+  }
+}
+
+// ---- y pass of planes too large for a block -----------------------------------------------
+//
+// An item is (slot, component, x, tile of kx kz columns), transformed in place like the x
+// pass's tiles, one component at a time: a tile's rows are then 128-byte runs where the x
+// pass, which needs all six components of a frequency, can hold 32.  Both outer stages touch
+// global memory from registers, so an element of a two-stage axis crosses shared memory twice
+// (the Stockham pass: five times, in two buffers).  Bound by HBM: the spectrum in and out.
+// With the z pass below, the 256^3 FP64 projection went from 2771 to 2399 us (3430 with no
+// register-tiled pass).
+#define DIFY_THREADS 128
+#define DIFY_MIN_BLOCKS(T) (sizeof(T) == 4 ? 7 : 4)
+
+template <typename T, bool INV>
+__global__ void __launch_bounds__(DIFY_THREADS, DIFY_MIN_BLOCKS(T))
+    dify_kernel(Grid<T> g, DifXPlan P, const SlotDev<T> *__restrict__ tab, SlotList list, int kry) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const DifAxis &Y = P.x;
+  const int ny = g.ny, hs = g.hs;
+  pdl_begin();
+  load_table<T>(reinterpret_cast<cplx<T> *>(smem_raw) + P.elems, g.twy, ny);
+  const SPtr<T> buf{smem_u32(smem_raw)}, tw = buf + P.elems;
+  const int per = 6 * g.nx * P.nkx;
+  pdl_wait();
+  const int n_items = list_items(list, per);
+  const int kxm = P.kx - 1, total0 = Y.m << P.lkx;
+  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+    const int ks = udiv(item, P.fd_items);
+    const int local = item - ks * per;
+    const int slot = list.ids[ks];
+    if (kry && slot_done(list.st + slot)) continue;
+    const int cx = udiv(local, P.fd_nkx), c = udiv(cx, g.fd_nx), x = cx - c * g.nx;
+    const int k0 = (local - cx * P.nkx) << P.lkx;
+    const int nk = min(P.kx, hs - k0);
+    cplx<T> *spec = reinterpret_cast<cplx<T> *>(tab[slot].spec) + c * g.S + (long long)x * ny * hs + k0;
+    __syncthreads();  // table ready; the previous item is done with the buffer
+    if constexpr (INV) {
+      // first inverse stage: frequencies j + nb q from global memory to their slots
+      DIF_RADIX(dif_last_radix(Y),
+        const int nb = ny / R;
+_Pragma("unroll 1")
+        for (int t = threadIdx.x; t < nb << P.lkx; t += blockDim.x) {
+          const int j = t >> P.lkx, col = t & kxm;
+          const cplx<T> *src = spec + j * hs + col;
+          const int step = nb * hs;
+          cplx<T> v[R];
+_Pragma("unroll")
+          for (int q = 0; q < R; ++q) v[q] = col < nk ? src[q * step] : mk<T>((T)0, (T)0);
+          dft<T, true, R>(v);
+          const SPtr<T> b = buf + dif_last_base(Y, j) + col;
+_Pragma("unroll")
+          for (int q = 0; q < R; ++q)
+            b.st(q * Y.a, q ? cmul<T>(v[q], dif_tw<T, true>(tw, q * j)) : v[q]);
+        }
+      )
+    } else {
+      DIF_RADIX(Y.r0,
+_Pragma("unroll 1")
+        for (int t = threadIdx.x; t < total0; t += blockDim.x) {
+          const int col = t & kxm, n = t >> P.lkx;
+          const cplx<T> *src = spec + n * hs + col;
+          const int step = Y.m * hs;
+          cplx<T> v[R];
+_Pragma("unroll")
+          for (int q = 0; q < R; ++q) v[q] = col < nk ? src[q * step] : mk<T>((T)0, (T)0);
+          dft<T, false, R>(v);
+          const SPtr<T> b = buf + n * Y.a + col;
+_Pragma("unroll")
+          for (int q = 0; q < R; ++q) b.st(q << P.lkx, q ? cmul<T>(v[q], tw.ld(q * n)) : v[q]);
+        }
+      )
+    }
+    __syncthreads();
+    if (Y.ns == 3) difx_middle<T, INV, 1>(buf, P, tw);
+    if constexpr (INV) {
+      DIF_RADIX(Y.r0,
+_Pragma("unroll 1")
+        for (int t = threadIdx.x; t < total0; t += blockDim.x) {
+          const int col = t & kxm, n = t >> P.lkx;
+          const SPtr<T> b = buf + n * Y.a + col;
+          cplx<T> v[R];
+_Pragma("unroll")
+          for (int q = 0; q < R; ++q) v[q] = b.ld(q << P.lkx);
+          dft<T, true, R>(v);
+          cplx<T> *dst = spec + n * hs + col;
+          const int step = Y.m * hs;
+          if (col < nk) {
+_Pragma("unroll")
+            for (int q = 0; q < R; ++q) dst[q * step] = v[q];
+          }
+        }
+      )
+    } else {
+      DIF_RADIX(dif_last_radix(Y),
+        const int nb = ny / R;
+_Pragma("unroll 1")
+        for (int t = threadIdx.x; t < nb << P.lkx; t += blockDim.x) {
+          const int j = t >> P.lkx, col = t & kxm;
+          const SPtr<T> b = buf + dif_last_base(Y, j) + col;
+          cplx<T> v[R];
+_Pragma("unroll")
+          for (int q = 0; q < R; ++q) v[q] = b.ld(q * Y.a);
+          dft<T, false, R>(v);
+          cplx<T> *dst = spec + j * hs + col;
+          const int step = nb * hs;
+          if (col < nk) {
+_Pragma("unroll")
+            for (int q = 0; q < R; ++q) dst[q * step] = v[q];
+          }
+        }
+      )
+    }
   }
 }
 
@@ -843,5 +957,192 @@ _Pragma("unroll")
       }
     )
     finish_inverse<TF, EPI>(S, acc0, acc1, acc2, local, per, red);
+  }
+}
+
+// ---- z pass of planes too large for a block -----------------------------------------------
+//
+// An item is (slot, tile of lz consecutive (x, y) lines, component pair).  The stages are the
+// plane passes' z stages; the split (or join) of the pair's two half spectra happens in
+// registers beside the access to global memory, so a line crosses shared memory twice a
+// two-stage axis and four times a three-stage one.  HBM-bound: the fields and the spectrum.
+#define DIFZ_THREADS 256
+#define DIFZ_MIN_BLOCKS(T) (sizeof(T) == 4 ? 4 : 2)
+
+struct DifZPlan {
+  int ok, lz, ntiles;  // lines a tile, tiles
+  DifPlane p;          // row layout and z axis (ls, elems, z)
+  FastDiv fd_items;
+};
+
+// Stage 1 of the tile's lines (three-stage axes).
+template <typename T, bool INV>
+__device__ __forceinline__ void difz_middle(SPtr<T> buf, const DifPlane &P, SPtr<T> tw, int nl) {
+  const int nb = P.z.r0 * P.z.r2;
+#pragma unroll 1
+  for (int t = threadIdx.x; t < nl * nb; t += blockDim.x) {
+    const int l = udiv(t, P.z.fd_nb1);
+    dif_stage1<T, INV>(buf + l * P.ls, P.z, t - l * nb, tw);
+  }
+  __syncthreads();
+}
+
+template <typename T>
+__global__ void __launch_bounds__(DIFZ_THREADS, DIFZ_MIN_BLOCKS(T))
+    dif_zfwd_kernel(Grid<T> g, DifZPlan P, const SlotDev<T> *__restrict__ tab, SlotList list,
+                    ExtIO<T> io, int kry) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const DifAxis &Z = P.p.z;
+  const int nz = g.nz, hs = g.hs, ls = P.p.ls;
+  const long long V = g.V, lines = (long long)g.nx * g.ny;
+  pdl_begin();
+  load_table<T>(reinterpret_cast<cplx<T> *>(smem_raw) + P.p.elems, g.twz, nz);
+  const SPtr<T> buf{smem_u32(smem_raw)}, tw = buf + P.p.elems;
+  const int per = 3 * P.ntiles;
+  pdl_wait();
+  const int n_items = list_items(list, per);
+  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+    const int ks = udiv(item, P.fd_items);
+    const int local = item - ks * per;
+    const int slot = list.ids[ks];
+    if (kry && slot_done(list.st + slot)) continue;
+    const SlotDev<T> &S = tab[slot];
+    const int tile = udiv(local, g.fd_3), p = local - 3 * tile;
+    const long long line0 = (long long)tile * P.lz;
+    const int nl = (int)min((long long)P.lz, lines - line0);
+    const T *src = (kry ? S.kr[6] : io.in) + 2 * p * V + line0 * nz;
+    __syncthreads();  // table ready; the previous item is done with the buffer
+    DIF_RADIX(Z.r0,
+_Pragma("unroll 1")
+      for (int t = threadIdx.x; t < nl * Z.m; t += blockDim.x) {
+        const int l = udiv(t, Z.fd_m), n = t - l * Z.m;
+        const T *s0 = src + (l * nz + n), *s1 = s0 + V;
+        cplx<T> v[R];
+_Pragma("unroll")
+        for (int q = 0; q < R; ++q) v[q] = mk<T>(s0[q * Z.m], s1[q * Z.m]);
+        dft<T, false, R>(v);
+        const SPtr<T> b = buf + l * ls + n * Z.a;
+_Pragma("unroll")
+        for (int q = 0; q < R; ++q) b.st(q, q ? cmul<T>(v[q], tw.ld(q * n)) : v[q]);
+      }
+    )
+    __syncthreads();
+    if (Z.ns == 3) difz_middle<T, false>(buf, P.p, tw, nl);
+    // last stage of frequencies j + nb q and their negatives, split into the two components
+    cplx<T> *spec = reinterpret_cast<cplx<T> *>(S.spec) + 2 * p * g.S + line0 * hs;
+    DIF_RADIX8(dif_last_radix(Z),
+      const int nb = nz / R, un = nb / 2 + 1;
+_Pragma("unroll 1")
+      for (int t = threadIdx.x; t < nl * un; t += blockDim.x) {
+        const int l = udiv(t, Z.fd_un), u = t - l * un;
+        const SPtr<T> row = buf + l * ls;
+        const SPtr<T> b1 = row + dif_last_base(Z, u), b2 = row + dif_last_base(Z, u == 0 ? 0 : nb - u);
+        cplx<T> v1[R], v2[R];
+_Pragma("unroll")
+        for (int q = 0; q < R; ++q) {
+          v1[q] = b1.ld(q * Z.a);
+          v2[q] = b2.ld(q * Z.a);
+        }
+        dft<T, false, R>(v1);
+        dft<T, false, R>(v2);
+        const bool self = u == 0 || 2 * u == nb;
+        cplx<T> *dst = spec + l * hs;
+_Pragma("unroll")
+        for (int q = 0; q < R; ++q) {
+          const cplx<T> Zk = v1[q], Zm = u == 0 ? v2[(R - q) % R] : v2[R - 1 - q];
+          const cplx<T> A = mk<T>((T)0.5 * (Zk.x + Zm.x), (T)0.5 * (Zk.y - Zm.y));
+          const cplx<T> B = mk<T>((T)0.5 * (Zk.y + Zm.y), (T)0.5 * (Zm.x - Zk.x));
+          const int kf = u + nb * q;
+          if (2 * kf < nz) {
+            dst[kf] = A;
+            dst[g.S + kf] = B;
+          } else if (2 * kf > nz && !self) {
+            dst[nz - kf] = cconj<T>(A);
+            dst[g.S + nz - kf] = cconj<T>(B);
+          }
+        }
+      }
+    )
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(DIFZ_THREADS, DIFZ_MIN_BLOCKS(T))
+    dif_zinv_kernel(Grid<T> g, DifZPlan P, const SlotDev<T> *__restrict__ tab, SlotList list,
+                    ExtIO<T> io, int kry) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const DifAxis &Z = P.p.z;
+  const int nz = g.nz, hs = g.hs, ls = P.p.ls;
+  const long long V = g.V, lines = (long long)g.nx * g.ny;
+  pdl_begin();
+  load_table<T>(reinterpret_cast<cplx<T> *>(smem_raw) + P.p.elems, g.twz, nz);
+  const SPtr<T> buf{smem_u32(smem_raw)}, tw = buf + P.p.elems;
+  const int per = 3 * P.ntiles;
+  pdl_wait();
+  const int n_items = list_items(list, per);
+  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+    const int ks = udiv(item, P.fd_items);
+    const int local = item - ks * per;
+    const int slot = list.ids[ks];
+    if (kry && slot_done(list.st + slot)) continue;
+    const SlotDev<T> &S = tab[slot];
+    const int tile = udiv(local, g.fd_3), p = local - 3 * tile;
+    const long long line0 = (long long)tile * P.lz;
+    const int nl = (int)min((long long)P.lz, lines - line0);
+    const cplx<T> *spec = reinterpret_cast<const cplx<T> *>(S.spec) + 2 * p * g.S + line0 * hs;
+    __syncthreads();  // table ready; the previous item is done with the buffer
+    // frequencies n' + m q of Z = A + iB and their negatives from the stored halves
+    // (Hermitian in z; the unstored Nyquist column is zero)
+    DIF_RADIX8(Z.r0,
+      const int m = Z.m, un = m / 2 + 1;
+_Pragma("unroll 1")
+      for (int t = threadIdx.x; t < nl * un; t += blockDim.x) {
+        const int l = udiv(t, Z.fd_un), n = t - l * un, n2 = n == 0 ? 0 : m - n;
+        const cplx<T> *src = spec + l * hs;
+        cplx<T> v1[R], v2[R];
+_Pragma("unroll")
+        for (int q = 0; q < R; ++q) {
+          const int kf = n + m * q;
+          const bool low = 2 * kf < nz, nyq = 2 * kf == nz;
+          const int kh = nyq ? 0 : (low ? kf : nz - kf);
+          const cplx<T> A = src[kh], B = src[g.S + kh];
+          const cplx<T> zl = mk<T>(A.x - B.y, A.y + B.x), zh = mk<T>(A.x + B.y, B.x - A.y);
+          v1[q] = nyq ? mk<T>((T)0, (T)0) : (low ? zl : zh);
+          v2[R - 1 - q] = nyq ? mk<T>((T)0, (T)0) : (low ? zh : zl);
+        }
+        dft<T, true, R>(v1);
+        const SPtr<T> b1 = buf + l * ls + n * Z.a, b2 = buf + l * ls + n2 * Z.a;
+_Pragma("unroll")
+        for (int q = 0; q < R; ++q)
+          b1.st(q, q ? cmul<T>(v1[q], dif_tw<T, true>(tw, q * n)) : v1[q]);
+        if (n != 0 && 2 * n != m) {
+          dft<T, true, R>(v2);
+_Pragma("unroll")
+          for (int q = 0; q < R; ++q)
+            b2.st(q, q ? cmul<T>(v2[q], dif_tw<T, true>(tw, q * n2)) : v2[q]);
+        }
+      }
+    )
+    __syncthreads();
+    if (Z.ns == 3) difz_middle<T, true>(buf, P.p, tw, nl);
+    T *out = (kry ? S.kr[6] : io.out) + 2 * p * V + line0 * nz;
+    DIF_RADIX(dif_last_radix(Z),
+      const int nb = nz / R;
+_Pragma("unroll 1")
+      for (int t = threadIdx.x; t < nl * nb; t += blockDim.x) {
+        const int l = udiv(t, Z.fd_nb), j = t - l * nb;
+        const SPtr<T> b = buf + l * ls + dif_last_base(Z, j);
+        cplx<T> v[R];
+_Pragma("unroll")
+        for (int q = 0; q < R; ++q) v[q] = b.ld(q * Z.a);
+        dft<T, true, R>(v);
+        T *d0 = out + (l * nz + j), *d1 = d0 + V;
+_Pragma("unroll")
+        for (int q = 0; q < R; ++q) {
+          d0[q * nb] = v[q].x;
+          d1[q * nb] = v[q].y;
+        }
+      }
+    )
   }
 }

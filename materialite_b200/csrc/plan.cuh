@@ -190,6 +190,8 @@ struct GridPlan {
   Grid<double> gd;
   DifPlane dplane[2][2];      // register-tiled passes: [0] float, [1] double; forward, inverse
   DifXPlan dx[2];
+  DifXPlan dy[2];             // passes of planes too large for a block: y (tiles as the x pass's)
+  DifZPlan dz[2][2];          // and z, forward and inverse
   size_t partial_doubles;     // reduction partials per slot
 };
 
@@ -394,21 +396,26 @@ static bool dif_axis(int n, unsigned first, unsigned last, DifAxis &A) {
 // takes 36 us there and 40 us in the register-tiled passes; 30 x 28 x 27 takes 52 and 41.
 #define DIF_MIN_PLANE 512
 
+// z axis and row layout of a forward (inv = false) or inverse pass.
+static bool dif_zrow(int nz, bool inv, DifPlane &P) {
+  memset(&P, 0, sizeof(P));
+  if (!dif_axis(nz, inv ? DIF_RADICES_PAIR : DIF_RADICES, inv ? DIF_RADICES : DIF_RADICES_PAIR, P.z))
+    return false;
+  P.z.a = P.z.r0 | 1;  // odd
+  P.z.b = 1;
+  P.ls = P.z.m * P.z.a;
+  const int nb = nz / (P.z.ns == 2 ? P.z.r1 : P.z.r2);
+  P.z.fd_un = make_fastdiv((uint32_t)((inv ? P.z.m : nb) / 2 + 1));
+  return true;
+}
+
 // Plan of the forward (inv = false) or inverse plane pass in one block's buffer (ok = 0 where
 // an axis has no plan or the plane is too large).
 template <typename T> static DifPlane dif_plane(int ny, int nz, int hs, bool inv) {
   DifPlane P;
-  memset(&P, 0, sizeof(P));
-  if (!dif_axis(nz, inv ? DIF_RADICES_PAIR : DIF_RADICES, inv ? DIF_RADICES : DIF_RADICES_PAIR, P.z) ||
-      !dif_axis(ny, DIF_RADICES, DIF_RADICES, P.y))
-    return P;
-  P.z.a = P.z.r0 | 1;  // odd
-  P.z.b = 1;
-  P.ls = P.z.m * P.z.a;
+  if (!dif_zrow(nz, inv, P) || !dif_axis(ny, DIF_RADICES, DIF_RADICES, P.y)) return P;
   // column (1, 0): the padding slot of n' = 0, or one more slot a row where there is none
   P.xslot = (P.z.r0 & 1) ? P.ls++ : P.z.r0;
-  const int nb = nz / (P.z.ns == 2 ? P.z.r1 : P.z.r2);
-  P.z.fd_un = make_fastdiv((uint32_t)((inv ? P.z.m : nb) / 2 + 1));
   P.elems = ny * P.ls;
   P.y.a = P.ls;
   P.y.b = P.y.m * P.ls;
@@ -455,6 +462,50 @@ template <typename T> static DifXPlan dif_xplan(int nx, int ny, int hs) {
   return P;
 }
 
+// y pass of planes too large for a block, one component a tile: 128-byte runs of a spectrum row,
+// halved (down to a 32-byte sector) while a tile exceeds 40 KB (five blocks an SM), while the
+// grid then has fewer than four tiles an SM, and while half of it is past the row's end.
+template <typename T> static DifXPlan dif_yplan(int nx, int ny, int hs) {
+  DifXPlan P;
+  memset(&P, 0, sizeof(P));
+  DifAxis &Y = P.x;
+  if (!dif_axis(ny, DIF_RADICES, DIF_RADICES, Y)) return P;
+  const int sector = 32 / (int)sizeof(cplx<T>);
+  const int w = 128 / (int)sizeof(cplx<T>);
+  P.kx = w;
+  auto layout = [&]() {
+    const int run = Y.r0 * P.kx;
+    Y.a = run + ((P.kx - run) % w + w) % w;
+    Y.b = P.kx;
+    P.cs = 0;
+    P.elems = Y.m * Y.a;
+    P.nkx = (hs + P.kx - 1) / P.kx;
+    return ((size_t)P.elems + ny) * sizeof(cplx<T>);
+  };
+  while (P.kx > sector && (layout() > 40 * 1024 || 6LL * nx * P.nkx < 4 * 148 || P.kx >= 2 * hs)) P.kx /= 2;
+  if (layout() > SMEM_LIMIT) return P;
+  while ((1 << P.lkx) < P.kx) ++P.lkx;
+  P.fd_mid = make_fastdiv((uint32_t)(Y.r0 * P.kx));
+  P.fd_r2 = make_fastdiv((uint32_t)Y.r2);
+  P.fd_items = make_fastdiv((uint32_t)(6 * nx * P.nkx));
+  P.fd_nkx = make_fastdiv((uint32_t)P.nkx);
+  P.ok = 1;
+  return P;
+}
+
+// z pass of such planes: tiles of about one radix-8 butterfly a thread and stage.
+template <typename T> static DifZPlan dif_zplan(long long lines, int nz, bool inv) {
+  DifZPlan P;
+  memset(&P, 0, sizeof(P));
+  if (!dif_zrow(nz, inv, P.p)) return P;
+  P.lz = (int)std::min<long long>(lines, std::max(1, 8 * DIFZ_THREADS / nz));
+  P.ntiles = (int)((lines + P.lz - 1) / P.lz);
+  P.p.elems = P.lz * P.p.ls;
+  P.fd_items = make_fastdiv((uint32_t)(3 * P.ntiles));
+  P.ok = ((size_t)P.p.elems + nz) * sizeof(cplx<T>) <= SMEM_LIMIT ? 1 : 0;
+  return P;
+}
+
 // x pass of a launch: the register-tiled one where nx has a plan for it (unless a tile shape
 // of the Stockham pass is asked for), else the Stockham one.
 template <typename T, typename TF, bool KRY>
@@ -469,6 +520,25 @@ static void launch_x(const GridPlan &p, const Grid<T> &g, long long cap, cudaStr
   const size_t sm = ((size_t)P.elems + p.nx) * sizeof(cplx<T>);
   const int grid = persistent_grid(k, DIFX_THREADS, sm, cap * P.nkx * p.ny, p.dev);
   launch_pdl(true, k, grid, DIFX_THREADS, sm, stream, g, P, reinterpret_cast<const SlotDev<T> *>(tab),
+             list, KRY ? 1 : 0);
+}
+
+// y pass of planes too large for a block: the register-tiled one where ny has a plan for it,
+// else the Stockham one.
+template <typename T, typename TF, bool INV, bool KRY>
+static void launch_y(const GridPlan &p, const Grid<T> &g, long long cap, cudaStream_t stream,
+                     const SlotDev<TF> *tab, SlotList list) {
+  const DifXPlan &P = p.dy[sizeof(T) == 8 ? 1 : 0];
+  if (!P.ok) {
+    const size_t sy = smem_y_bytes<T>(p.ky, p.ny);
+    auto ky = ypass_kernel<T, TF, INV, KRY>;
+    ky<<<persistent_grid(ky, SSFFT_THREADS, sy, cap * items_y(g), p.dev), SSFFT_THREADS, sy, stream>>>(g, tab, list);
+    return;
+  }
+  auto k = dify_kernel<T, INV>;
+  const size_t sm = ((size_t)P.elems + p.ny) * sizeof(cplx<T>);
+  const int grid = persistent_grid(k, DIFY_THREADS, sm, cap * 6 * p.nx * P.nkx, p.dev);
+  launch_pdl(true, k, grid, DIFY_THREADS, sm, stream, g, P, reinterpret_cast<const SlotDev<T> *>(tab),
              list, KRY ? 1 : 0);
 }
 
@@ -578,6 +648,15 @@ static int plan_create(GridPlan &p, const ssfft_config *cfg, cudaStream_t stream
   if (p.ny * p.nz >= DIF_MIN_PLANE && env_int("SSFFT_XPASS_KX") <= 0 && env_int("SSFFT_XPASS_THREADS") <= 0) {
     p.dx[0] = dif_xplan<float>(p.nx, p.ny, p.gd.hs);
     p.dx[1] = dif_xplan<double>(p.nx, p.ny, p.gd.hs);
+    // SSFFT_NO_PLANE keeps the Stockham five-pass kernels
+    if (p.use_plane) {
+      p.dy[0] = dif_yplan<float>(p.nx, p.ny, p.gd.hs);
+      p.dy[1] = dif_yplan<double>(p.nx, p.ny, p.gd.hs);
+      for (int d = 0; d < 2; ++d) {
+        p.dz[0][d] = dif_zplan<float>((long long)p.nx * p.ny, p.nz, d == 1);
+        p.dz[1][d] = dif_zplan<double>((long long)p.nx * p.ny, p.nz, d == 1);
+      }
+    }
   }
   // items of one slot per reduction, times the values each stores
   const Grid<double> &g = p.gd;
@@ -668,6 +747,16 @@ template <typename T, typename TF> static int set_kernel_attrs(const GridPlan &p
     }
   }
   if (p.dplane[k][0].ok && p.dplane[k][1].ok) return dif_plane_attrs<T, TF>();
+  if (p.dy[k].ok) {
+    CKR((smem_attr(dify_kernel<T, false>, m)));
+    CKR((smem_attr(dify_kernel<T, true>, m)));
+  }
+  if constexpr (sizeof(T) == sizeof(TF)) {
+    if (p.dz[k][0].ok && p.dz[k][1].ok) {
+      CKR(smem_attr(dif_zfwd_kernel<T>, m));
+      CKR(smem_attr(dif_zinv_kernel<T>, m));
+    }
+  }
   CKR(smem_attr(zfwd_kernel<T, TF, PRO_INPUT>, m));
   CKR(smem_attr(zfwd_kernel<T, TF, PRO_RESIDUAL>, m));
   CKR(smem_attr(zfwd_kernel<T, TF, PRO_REPROJECT>, m));
@@ -1170,22 +1259,44 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
     if (c.launches) *c.launches += 3;
   } else {
     const size_t sz = smem_z_bytes<T>(p.lz, p.nz);
-    const size_t sy = smem_y_bytes<T>(p.ky, p.ny);
     const long long itz = (long long)c.cap * items_z(g);
-    const long long ity = (long long)c.cap * items_y(g);
-    auto kz = zfwd_kernel<T, TF, PRO>;
-    kz<<<persistent_grid(kz, SSFFT_THREADS, sz, itz, dev), SSFFT_THREADS, sz, c.stream>>>(g, tab, c.list, io);
+    // register-tiled z passes where nz has a plan and a pass only moves planes (the residual
+    // and the re-projection, one each a Newton iteration, keep the Stockham ones)
+    const DifZPlan *dz = p.dz[sizeof(T) == 8 ? 1 : 0];
+    constexpr bool PLANES = sizeof(T) == sizeof(TF) && (PRO == PRO_INPUT || PRO == PRO_TAU) &&
+                            (EPI == EPI_STORE || EPI == EPI_PTAU);
+    const bool dif_z = PLANES && dz[0].ok && dz[1].ok;
+    if constexpr (PLANES) {
+      if (dif_z) {
+        auto k = dif_zfwd_kernel<T>;
+        const size_t sm = ((size_t)dz[0].p.elems + p.nz) * sizeof(cplx<T>);
+        const int grid = persistent_grid(k, DIFZ_THREADS, sm, (long long)c.cap * 3 * dz[0].ntiles, dev);
+        launch_pdl(KRY, k, grid, DIFZ_THREADS, sm, c.stream, g, dz[0], tab, c.list, io, KRY ? 1 : 0);
+      }
+    }
+    if (!dif_z) {
+      auto kz = zfwd_kernel<T, TF, PRO>;
+      kz<<<persistent_grid(kz, SSFFT_THREADS, sz, itz, dev), SSFFT_THREADS, sz, c.stream>>>(g, tab, c.list, io);
+    }
     rec(1);
-    auto ky = ypass_kernel<T, TF, false, KRY>;
-    ky<<<persistent_grid(ky, SSFFT_THREADS, sy, ity, dev), SSFFT_THREADS, sy, c.stream>>>(g, tab, c.list);
+    launch_y<T, TF, false, KRY>(p, g, c.cap, c.stream, tab, c.list);
     rec(2);
     launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list);
     rec(3);
-    auto kyi = ypass_kernel<T, TF, true, KRY>;
-    kyi<<<persistent_grid(kyi, SSFFT_THREADS, sy, ity, dev), SSFFT_THREADS, sy, c.stream>>>(g, tab, c.list);
+    launch_y<T, TF, true, KRY>(p, g, c.cap, c.stream, tab, c.list);
     rec(4);
-    auto kzi = zinv_kernel<T, TF, EPI>;
-    kzi<<<persistent_grid(kzi, SSFFT_THREADS, sz, itz, dev), SSFFT_THREADS, sz, c.stream>>>(g, tab, c.list, io);
+    if constexpr (PLANES) {
+      if (dif_z) {
+        auto k = dif_zinv_kernel<T>;
+        const size_t sm = ((size_t)dz[1].p.elems + p.nz) * sizeof(cplx<T>);
+        const int grid = persistent_grid(k, DIFZ_THREADS, sm, (long long)c.cap * 3 * dz[1].ntiles, dev);
+        launch_pdl(true, k, grid, DIFZ_THREADS, sm, c.stream, g, dz[1], tab, c.list, io, KRY ? 1 : 0);
+      }
+    }
+    if (!dif_z) {
+      auto kzi = zinv_kernel<T, TF, EPI>;
+      kzi<<<persistent_grid(kzi, SSFFT_THREADS, sz, itz, dev), SSFFT_THREADS, sz, c.stream>>>(g, tab, c.list, io);
+    }
     rec(5);
     if (c.launches) *c.launches += 5;
   }
