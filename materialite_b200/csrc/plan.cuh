@@ -396,6 +396,8 @@ static bool dif_axis(int n, unsigned first, unsigned last, DifAxis &A) {
 // takes 36 us there and 40 us in the register-tiled passes; 30 x 28 x 27 takes 52 and 41.
 #define DIF_MIN_PLANE 512
 
+static int dif_last_radix_host(const DifAxis &A) { return A.ns == 2 ? A.r1 : A.r2; }
+
 // z axis and row layout of a forward (inv = false) or inverse pass.
 static bool dif_zrow(int nz, bool inv, DifPlane &P) {
   memset(&P, 0, sizeof(P));
@@ -404,7 +406,7 @@ static bool dif_zrow(int nz, bool inv, DifPlane &P) {
   P.z.a = P.z.r0 | 1;  // odd
   P.z.b = 1;
   P.ls = P.z.m * P.z.a;
-  const int nb = nz / (P.z.ns == 2 ? P.z.r1 : P.z.r2);
+  const int nb = nz / dif_last_radix_host(P.z);
   P.z.fd_un = make_fastdiv((uint32_t)((inv ? P.z.m : nb) / 2 + 1));
   return true;
 }
@@ -493,12 +495,16 @@ template <typename T> static DifXPlan dif_yplan(int nx, int ny, int hs) {
   return P;
 }
 
-// z pass of such planes: tiles of about one radix-8 butterfly a thread and stage.
+// z pass of such planes: tiles of as many lines as give each thread one pair of butterflies in
+// the paired stage (the slowest: two lines' registers a thread), of at most 100 KB in double and
+// 50 KB in float (as many blocks an SM as the registers allow).
 template <typename T> static DifZPlan dif_zplan(long long lines, int nz, bool inv) {
   DifZPlan P;
   memset(&P, 0, sizeof(P));
   if (!dif_zrow(nz, inv, P.p)) return P;
-  P.lz = (int)std::min<long long>(lines, std::max(1, 8 * DIFZ_THREADS / nz));
+  const int un = (inv ? P.p.z.m : nz / dif_last_radix_host(P.p.z)) / 2 + 1;
+  const int most = (sizeof(T) == 8 ? 100 : 50) * 1024 / (int)(P.p.ls * sizeof(cplx<T>));
+  P.lz = (int)std::min<long long>(lines, std::max(1, std::min(DIFZ_THREADS / un, most)));
   P.ntiles = (int)((lines + P.lz - 1) / P.lz);
   P.p.elems = P.lz * P.p.ls;
   P.fd_items = make_fastdiv((uint32_t)(3 * P.ntiles));
@@ -648,8 +654,8 @@ static int plan_create(GridPlan &p, const ssfft_config *cfg, cudaStream_t stream
   if (p.ny * p.nz >= DIF_MIN_PLANE && env_int("SSFFT_XPASS_KX") <= 0 && env_int("SSFFT_XPASS_THREADS") <= 0) {
     p.dx[0] = dif_xplan<float>(p.nx, p.ny, p.gd.hs);
     p.dx[1] = dif_xplan<double>(p.nx, p.ny, p.gd.hs);
-    // SSFFT_NO_PLANE keeps the Stockham five-pass kernels
-    if (p.use_plane) {
+    // SSFFT_NO_PLANE keeps the Stockham five-pass kernels, SSFFT_CLUSTER the cluster passes
+    if (p.use_plane && env_int("SSFFT_CLUSTER") <= 0) {
       p.dy[0] = dif_yplan<float>(p.nx, p.ny, p.gd.hs);
       p.dy[1] = dif_yplan<double>(p.nx, p.ny, p.gd.hs);
       for (int d = 0; d < 2; ++d) {
@@ -1204,12 +1210,22 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
   };
   const int dev = p.dev;
   const DifPlane *dp = p.dplane[sizeof(T) == 8 ? 1 : 0];
+  // register-tiled z passes where nz has a plan and a pass only moves planes (the residual
+  // and the re-projection, one each a Newton iteration, keep the Stockham ones)
+  const DifZPlan *dz = p.dz[sizeof(T) == 8 ? 1 : 0];
+  constexpr bool PLANES = sizeof(T) == sizeof(TF) && (PRO == PRO_INPUT || PRO == PRO_TAU) &&
+                          (EPI == EPI_STORE || EPI == EPI_PTAU);
+  const bool dif_z = PLANES && dz[0].ok && dz[1].ok;
+  // Five register-tiled passes beat three on clusters wherever both run (projections, us,
+  // clusters / five passes: 128^3 FP64 451 / 305, 64 x 128 x 144 FP64 280 / 190, 160^3 FP64
+  // 1203 / 615, 192^3 FP64 1725 / 1007 and float 830 / 580, 256^3 float 2201 / 1262).
+  const bool five = dif_z && p.dy[sizeof(T) == 8 ? 1 : 0].ok;
   rec(0);
   if (dp[0].ok && dp[1].ok) {
     launch_dif_planes<T, TF, PRO, EPI>(c, tab, io, dp, rec);
     rec(5);
     if (c.launches) *c.launches += 3;
-  } else if (const int C = cluster_size<T>(p)) {
+  } else if (const int C = five ? 0 : cluster_size<T>(p)) {
     const ClusterGeo q = cluster_geo<T>(p, C);
     const size_t sp = smem_cplane_bytes<T>(p.ny, p.nz, g.hs, C);
     const long long it = (long long)c.cap * items_plane(g);
@@ -1260,12 +1276,6 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
   } else {
     const size_t sz = smem_z_bytes<T>(p.lz, p.nz);
     const long long itz = (long long)c.cap * items_z(g);
-    // register-tiled z passes where nz has a plan and a pass only moves planes (the residual
-    // and the re-projection, one each a Newton iteration, keep the Stockham ones)
-    const DifZPlan *dz = p.dz[sizeof(T) == 8 ? 1 : 0];
-    constexpr bool PLANES = sizeof(T) == sizeof(TF) && (PRO == PRO_INPUT || PRO == PRO_TAU) &&
-                            (EPI == EPI_STORE || EPI == EPI_PTAU);
-    const bool dif_z = PLANES && dz[0].ok && dz[1].ok;
     if constexpr (PLANES) {
       if (dif_z) {
         auto k = dif_zfwd_kernel<T>;
