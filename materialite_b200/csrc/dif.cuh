@@ -1,5 +1,6 @@
 // Register-tiled transform passes for axes whose length factors into two or three radices up
-// to 16 (primes up to 7): the x pass with Gamma-hat, and the fused z and y passes of one x plane.
+// to 16 (primes up to 7): the x pass with Gamma-hat, the fused z and y passes of one x plane, and
+// separate z and y passes for planes too large for a block.
 //
 // Every line is transformed in place in one shared-memory buffer by decimation in frequency.
 // A length N = r_0 r_1 .. r_s line is viewed as digits: stage 0 takes, for each
@@ -243,8 +244,14 @@ struct DifXPlan {
   FastDiv fd_mid, fd_r2, fd_items, fd_nkx;
 };
 
+// MB blocks an SM: five in float.  In double three (96 registers), which hide more of the
+// latency than two (168), up to 200 points along x, and two for longer lines, whose tiles of
+// 46 KB and more are in flight enough at two blocks and whose radix-16 stages spill at three.
+// Projections in FP64, us, two / three blocks: 45 x 50 x 63 47.3 / 44.7, 96 x 80 x 60 82.0 / 76.8,
+// 135 x 175 x 189 771 / 723, 128^3 305 / 297, 192^3 1007 / 1008, 200 x 225 x 64 469 / 460;
+// 240 x 96 x 250 977 / 1051, 256^3 2177 / 2320.
 #define DIFX_THREADS 192
-#define DIFX_MIN_BLOCKS(T) (sizeof(T) == 4 ? 5 : 2)
+#define DIFX_THREE_MOST 200
 
 // Gamma-hat of one frequency on the six components m[], with t = (t0, t1, t2) = tan(pi f) not
 // normalised: s = t / |t|^2, u = T t, O = s (x) u + u (x) s - (s . u) s (x) t, times the
@@ -341,8 +348,8 @@ _Pragma("unroll")
   __syncthreads();
 }
 
-template <typename T>
-__global__ void __launch_bounds__(DIFX_THREADS, DIFX_MIN_BLOCKS(T))
+template <typename T, int MB>
+__global__ void __launch_bounds__(DIFX_THREADS, MB)
     difx_kernel(Grid<T> g, DifXPlan P, const SlotDev<T> *__restrict__ tab, SlotList list, int kry) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const DifAxis &X = P.x;

@@ -512,6 +512,15 @@ template <typename T> static DifZPlan dif_zplan(long long lines, int nz, bool in
   return P;
 }
 
+// The register-tiled x pass of lines of nx points.
+template <typename T>
+static void (*difx_of(int nx))(Grid<T>, DifXPlan, const SlotDev<T> *, SlotList, int) {
+  if constexpr (sizeof(T) == 4)
+    return difx_kernel<T, 5>;
+  else
+    return nx <= DIFX_THREE_MOST ? difx_kernel<T, 3> : difx_kernel<T, 2>;
+}
+
 // x pass of a launch: the register-tiled one where nx has a plan for it (unless a tile shape
 // of the Stockham pass is asked for), else the Stockham one.
 template <typename T, typename TF, bool KRY>
@@ -522,7 +531,7 @@ static void launch_x(const GridPlan &p, const Grid<T> &g, long long cap, cudaStr
     launch_xpass<T, TF, KRY>(g, smem_x_bytes<T>(g.kx, p.nx), cap * items_x(g), p.dev, stream, tab, list);
     return;
   }
-  auto k = difx_kernel<T>;
+  auto k = difx_of<T>(p.nx);
   const size_t sm = ((size_t)P.elems + p.nx) * sizeof(cplx<T>);
   const int grid = persistent_grid(k, DIFX_THREADS, sm, cap * P.nkx * p.ny, p.dev);
   launch_pdl(true, k, grid, DIFX_THREADS, sm, stream, g, P, reinterpret_cast<const SlotDev<T> *>(tab),
@@ -741,7 +750,7 @@ template <typename T, typename TF> static int set_kernel_attrs(const GridPlan &p
   const int k = sizeof(T) == 8 ? 1 : 0;
   if constexpr (sizeof(T) == sizeof(TF)) CKR(smem_attr(constitutive_kernel<T>, (int)constitutive_smem_bytes()));
   if (p.dx[k].ok) {
-    CKR(smem_attr(difx_kernel<T>, m));
+    CKR(smem_attr(difx_of<T>(p.nx), m));
   } else {
     CKR((smem_attr(xpass_kernel<T, TF, false>, m)));
     CKR((smem_attr(xpass_kernel<T, TF, true>, m)));
