@@ -775,7 +775,7 @@ def accuracy_mode(args, w):
 
 
 # DRAM read + write bytes of one steady-state launch of each Krylov kernel on plain128
-# (128^3, mixed precision, three-pass cluster path), from one-launch ncu captures of
+# (128^3, mixed precision; the transforms as cluster passes), from one-launch ncu captures of
 # `--mode kernels --workload plain128` (profiles/krylov_kernels_plain128.md).  The update
 # kernel reads 260.1 MB and writes 154.2 MB against 461 MB algorithmic: part of its writes
 # are still in L2 when it ends.
