@@ -9,10 +9,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
-#include <mutex>
 #include <string>
-#include <utility>
 #include <vector>
 
 #include "../../include/ssfft.h"
@@ -22,23 +19,9 @@
 #include "fft.cuh"
 #include "fields.cuh"
 #include "krylov.cuh"
+#include "launch.cuh"
 #include "projector.cuh"
 #include "slots.cuh"
-
-int ssfft_internal_fail(int code, const std::string &msg);
-
-#define CK(call)                                                                          \
-  do {                                                                                    \
-    cudaError_t e_ = (call);                                                              \
-    if (e_ != cudaSuccess)                                                                \
-      return ssfft_internal_fail(SSFFT_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
-  } while (0)
-
-#define CKR(expr)           \
-  do {                      \
-    int r_ = (expr);        \
-    if (r_ != 0) return r_; \
-  } while (0)
 
 #define ALLOC(ptr, bytes)                                                                 \
   do {                                                                                    \
@@ -51,122 +34,6 @@ int ssfft_internal_fail(int code, const std::string &msg);
   } while (0)
 
 static int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
-
-// ---------------------------------------------------------------------------------------
-// persistent grids
-// ---------------------------------------------------------------------------------------
-// Blocks of a persistent launch: as many as are resident at once on the device (occupancy
-// x SMs), but no more than there are items.
-struct OccKey {
-  const void *f;
-  int threads;
-  size_t smem;
-  int dev;
-  int cluster;  // 0: blocks; C: clusters of C blocks
-  bool operator<(const OccKey &o) const {
-    if (f != o.f) return f < o.f;
-    if (threads != o.threads) return threads < o.threads;
-    if (smem != o.smem) return smem < o.smem;
-    if (dev != o.dev) return dev < o.dev;
-    return cluster < o.cluster;
-  }
-};
-
-static std::mutex g_occ_mutex;
-static std::map<OccKey, int> g_occ;
-
-template <typename F> static int resident_blocks(F f, int threads, size_t smem, int dev) {
-  const OccKey key{(const void *)f, threads, smem, dev, 0};
-  {
-    std::lock_guard<std::mutex> lk(g_occ_mutex);
-    auto it = g_occ.find(key);
-    if (it != g_occ.end()) return it->second;
-  }
-  int per_sm = 0, sms = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess)
-    per_sm = 1;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-  cudaGetLastError();
-  const int n = std::max(1, per_sm) * std::max(1, sms);
-  std::lock_guard<std::mutex> lk(g_occ_mutex);
-  g_occ[key] = n;
-  return n;
-}
-
-template <typename F>
-static int persistent_grid(F f, int threads, size_t smem, long long items, int dev) {
-  return (int)std::max(1LL, std::min<long long>(items, resident_blocks(f, threads, smem, dev)));
-}
-
-// Clusters of C blocks resident at once (a cluster must fit the SMs of one GPC).
-template <typename... A>
-static int resident_clusters(void (*f)(A...), int C, int threads, size_t smem, int dev) {
-  const OccKey key{(const void *)f, threads, smem, dev, C};
-  {
-    std::lock_guard<std::mutex> lk(g_occ_mutex);
-    auto it = g_occ.find(key);
-    if (it != g_occ.end()) return it->second;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = C;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(C);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, f, &cfg) != cudaSuccess || n < 1) n = 1;
-  cudaGetLastError();
-  std::lock_guard<std::mutex> lk(g_occ_mutex);
-  g_occ[key] = n;
-  return n;
-}
-
-// Persistent launch of a cluster kernel of `threads` threads a block: as many clusters as
-// are resident at once, but no more than there are items.
-template <typename... P, typename... A>
-static int launch_clustered(void (*f)(P...), int C, int threads, size_t smem, long long items,
-                            int dev, cudaStream_t stream, A &&...args) {
-  const int ncl = (int)std::max(1LL, std::min<long long>(items, resident_clusters(f, C, threads, smem, dev)));
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = C;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)(ncl * C));
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, f, std::forward<A>(args)...);
-  if (e != cudaSuccess)
-    return ssfft_internal_fail(SSFFT_E_CUDA, std::string("cluster launch: ") + cudaGetErrorString(e));
-  return 0;
-}
-
-// Launch of a kernel that calls pdl_wait(): with `pdl`, it may start while the kernel before it
-// in the stream still runs.
-template <typename... P, typename... A>
-static void launch_pdl(bool pdl, void (*f)(P...), int grid, int threads, size_t smem,
-                       cudaStream_t stream, A &&...args) {
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = at;
-  cfg.numAttrs = pdl ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, f, std::forward<A>(args)...);
-}
 
 // ---------------------------------------------------------------------------------------
 // grid plan
@@ -321,23 +188,22 @@ template <typename T> static int xpass_threads() {
 }
 
 template <typename T, typename TF, bool KRY>
-static void launch_xpass(const Grid<T> &g, size_t sx, long long items, int dev,
+static int launch_xpass(const Grid<T> &g, size_t sx, long long items, int dev,
                          cudaStream_t stream, const SlotDev<TF> *tab, SlotList list) {
   const int pt = xpass_threads<T>();
   if constexpr (sizeof(T) == 4) {
     if (pt == 384) {
       auto k = xpass_kernel<T, TF, KRY, 384>;
-      k<<<persistent_grid(k, 384, sx, items, dev), 384, sx, stream>>>(g, tab, list);
-      return;
+      return launch_kernel(false, k, persistent_grid(k, 384, sx, items, dev), 384, sx, stream, g, tab, list);
     }
     if (pt == 192) {
       auto k = xpass_kernel<T, TF, KRY, 192>;
-      k<<<persistent_grid(k, 192, sx, items, dev), 192, sx, stream>>>(g, tab, list);
-      return;
+      return launch_kernel(false, k, persistent_grid(k, 192, sx, items, dev), 192, sx, stream, g, tab, list);
     }
   }
   auto k = xpass_kernel<T, TF, KRY>;
-  k<<<persistent_grid(k, XPASS_THREADS, sx, items, dev), XPASS_THREADS, sx, stream>>>(g, tab, list);
+  return launch_kernel(false, k, persistent_grid(k, XPASS_THREADS, sx, items, dev), XPASS_THREADS, sx,
+                       stream, g, tab, list);
 }
 
 // The projection runs as three passes (z and y fused, in one block or one cluster).
@@ -524,37 +390,35 @@ static void (*difx_of(int nx))(Grid<T>, DifXPlan, const SlotDev<T> *, SlotList, 
 // x pass of a launch: the register-tiled one where nx has a plan for it (unless a tile shape
 // of the Stockham pass is asked for), else the Stockham one.
 template <typename T, typename TF, bool KRY>
-static void launch_x(const GridPlan &p, const Grid<T> &g, long long cap, cudaStream_t stream,
+static int launch_x(const GridPlan &p, const Grid<T> &g, long long cap, cudaStream_t stream,
                      const SlotDev<TF> *tab, SlotList list) {
   const DifXPlan &P = p.dx[sizeof(T) == 8 ? 1 : 0];
-  if (!P.ok) {
-    launch_xpass<T, TF, KRY>(g, smem_x_bytes<T>(g.kx, p.nx), cap * items_x(g), p.dev, stream, tab, list);
-    return;
-  }
+  if (!P.ok)
+    return launch_xpass<T, TF, KRY>(g, smem_x_bytes<T>(g.kx, p.nx), cap * items_x(g), p.dev, stream, tab, list);
   auto k = difx_of<T>(p.nx);
   const size_t sm = ((size_t)P.elems + p.nx) * sizeof(cplx<T>);
   const int grid = persistent_grid(k, DIFX_THREADS, sm, cap * P.nkx * p.ny, p.dev);
-  launch_pdl(true, k, grid, DIFX_THREADS, sm, stream, g, P, reinterpret_cast<const SlotDev<T> *>(tab),
-             list, KRY ? 1 : 0);
+  return launch_kernel(true, k, grid, DIFX_THREADS, sm, stream, g, P,
+                       reinterpret_cast<const SlotDev<T> *>(tab), list, KRY ? 1 : 0);
 }
 
 // y pass of planes too large for a block: the register-tiled one where ny has a plan for it,
 // else the Stockham one.
 template <typename T, typename TF, bool INV, bool KRY>
-static void launch_y(const GridPlan &p, const Grid<T> &g, long long cap, cudaStream_t stream,
+static int launch_y(const GridPlan &p, const Grid<T> &g, long long cap, cudaStream_t stream,
                      const SlotDev<TF> *tab, SlotList list) {
   const DifXPlan &P = p.dy[sizeof(T) == 8 ? 1 : 0];
   if (!P.ok) {
     const size_t sy = smem_y_bytes<T>(p.ky, p.ny);
     auto ky = ypass_kernel<T, TF, INV, KRY>;
-    ky<<<persistent_grid(ky, SSFFT_THREADS, sy, cap * items_y(g), p.dev), SSFFT_THREADS, sy, stream>>>(g, tab, list);
-    return;
+    return launch_kernel(false, ky, persistent_grid(ky, SSFFT_THREADS, sy, cap * items_y(g), p.dev),
+                         SSFFT_THREADS, sy, stream, g, tab, list);
   }
   auto k = dify_kernel<T, INV>;
   const size_t sm = ((size_t)P.elems + p.ny) * sizeof(cplx<T>);
   const int grid = persistent_grid(k, DIFY_THREADS, sm, cap * 6 * p.nx * P.nkx, p.dev);
-  launch_pdl(true, k, grid, DIFY_THREADS, sm, stream, g, P, reinterpret_cast<const SlotDev<T> *>(tab),
-             list, KRY ? 1 : 0);
+  return launch_kernel(true, k, grid, DIFY_THREADS, sm, stream, g, P,
+                       reinterpret_cast<const SlotDev<T> *>(tab), list, KRY ? 1 : 0);
 }
 
 static int validate_config(const ssfft_config *cfg) {
@@ -1172,7 +1036,7 @@ struct LaunchCtx {
 
 // The register-tiled plane passes of one projection around the x pass.
 template <typename T, typename TF, int PRO, int EPI, typename REC>
-static void launch_dif_planes(const LaunchCtx &c, const SlotDev<TF> *tab, const ExtIO<TF> &io,
+static int launch_dif_planes(const LaunchCtx &c, const SlotDev<TF> *tab, const ExtIO<TF> &io,
                               const DifPlane *PP, const REC &rec) {
   const DifPlane &P = PP[0], &Q = PP[1];
   constexpr bool KRY = PRO == PRO_TAU;
@@ -1185,22 +1049,22 @@ static void launch_dif_planes(const LaunchCtx &c, const SlotDev<TF> *tab, const 
   if constexpr (PRO == PRO_RESIDUAL) {
     // the residual reads the stress alone, which is double for either storage type
     auto kf = dif_zyfwd_kernel<double, double, DIF_RESIDUAL>;
-    launch_pdl(false, kf, persistent_grid(kf, pt, sp, it, p.dev), pt, sp, c.stream, g, P,
-               reinterpret_cast<const SlotDev<double> *>(tab), c.list, ExtIO<double>{}, (int)PRO);
+    CKR(launch_kernel(false, kf, persistent_grid(kf, pt, sp, it, p.dev), pt, sp, c.stream, g, P,
+                      reinterpret_cast<const SlotDev<double> *>(tab), c.list, ExtIO<double>{}, (int)PRO));
   } else {
     auto kf = dif_zyfwd_kernel<T, TF, DIF_PLANES>;
-    launch_pdl(KRY, kf, persistent_grid(kf, pt, sp, it, p.dev), pt, sp, c.stream, g, P, tab, c.list,
-               io, (int)PRO);
+    CKR(launch_kernel(KRY, kf, persistent_grid(kf, pt, sp, it, p.dev), pt, sp, c.stream, g, P, tab,
+                      c.list, io, (int)PRO));
   }
   rec(1);
   rec(2);
-  launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list);
+  CKR((launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list)));
   rec(3);
   rec(4);
   constexpr int KIND = EPI == EPI_RESIDUAL ? DIF_RESIDUAL : (EPI == EPI_REPROJECT ? DIF_REPROJECT : DIF_PLANES);
   auto ki = dif_yzinv_kernel<T, TF, KIND>;
-  launch_pdl(true, ki, persistent_grid(ki, pt, sq, it, p.dev), pt, sq, c.stream, g, Q, tab, c.list, io,
-             (int)EPI);
+  return launch_kernel(true, ki, persistent_grid(ki, pt, sq, it, p.dev), pt, sq, c.stream, g, Q, tab,
+                       c.list, io, (int)EPI);
 }
 
 // The passes of one projection.  ev (optional, 6 events) is recorded before the first pass
@@ -1231,7 +1095,7 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
   const bool five = dif_z && p.dy[sizeof(T) == 8 ? 1 : 0].ok;
   rec(0);
   if (dp[0].ok && dp[1].ok) {
-    launch_dif_planes<T, TF, PRO, EPI>(c, tab, io, dp, rec);
+    CKR((launch_dif_planes<T, TF, PRO, EPI>(c, tab, io, dp, rec)));
     rec(5);
     if (c.launches) *c.launches += 3;
   } else if (const int C = five ? 0 : cluster_size<T>(p)) {
@@ -1247,7 +1111,7 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
       CKR(launch_clustered(zyfwd_cl_kernel<T, TF, PRO, 512>, C, 512, sp, it, dev, c.stream, g, q, tab, c.list, io));
     rec(1);
     rec(2);
-    launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list);
+    CKR((launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list)));
     rec(3);
     rec(4);
     if (pt == 1024)
@@ -1263,22 +1127,22 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
     const long long it = (long long)c.cap * items_plane(g);
     if (plane_threads<T>(p) == 1024) {
       auto kf = zyfwd_kernel<T, TF, PRO, 1024>;
-      kf<<<persistent_grid(kf, 1024, sp, it, dev), 1024, sp, c.stream>>>(g, tab, c.list, io);
+      CKR(launch_kernel(false, kf, persistent_grid(kf, 1024, sp, it, dev), 1024, sp, c.stream, g, tab, c.list, io));
     } else {
       auto kf = zyfwd_kernel<T, TF, PRO, 512>;
-      kf<<<persistent_grid(kf, 512, sp, it, dev), 512, sp, c.stream>>>(g, tab, c.list, io);
+      CKR(launch_kernel(false, kf, persistent_grid(kf, 512, sp, it, dev), 512, sp, c.stream, g, tab, c.list, io));
     }
     rec(1);
     rec(2);
-    launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list);
+    CKR((launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list)));
     rec(3);
     rec(4);
     if (plane_threads<T>(p) == 1024) {
       auto ki = yzinv_kernel<T, TF, EPI, 1024>;
-      ki<<<persistent_grid(ki, 1024, sp, it, dev), 1024, sp, c.stream>>>(g, tab, c.list, io);
+      CKR(launch_kernel(false, ki, persistent_grid(ki, 1024, sp, it, dev), 1024, sp, c.stream, g, tab, c.list, io));
     } else {
       auto ki = yzinv_kernel<T, TF, EPI, 512>;
-      ki<<<persistent_grid(ki, 512, sp, it, dev), 512, sp, c.stream>>>(g, tab, c.list, io);
+      CKR(launch_kernel(false, ki, persistent_grid(ki, 512, sp, it, dev), 512, sp, c.stream, g, tab, c.list, io));
     }
     rec(5);
     if (c.launches) *c.launches += 3;
@@ -1290,31 +1154,33 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
         auto k = dif_zfwd_kernel<T>;
         const size_t sm = ((size_t)dz[0].p.elems + p.nz) * sizeof(cplx<T>);
         const int grid = persistent_grid(k, DIFZ_THREADS, sm, (long long)c.cap * 3 * dz[0].ntiles, dev);
-        launch_pdl(KRY, k, grid, DIFZ_THREADS, sm, c.stream, g, dz[0], tab, c.list, io, KRY ? 1 : 0);
+        CKR(launch_kernel(KRY, k, grid, DIFZ_THREADS, sm, c.stream, g, dz[0], tab, c.list, io, KRY ? 1 : 0));
       }
     }
     if (!dif_z) {
       auto kz = zfwd_kernel<T, TF, PRO>;
-      kz<<<persistent_grid(kz, SSFFT_THREADS, sz, itz, dev), SSFFT_THREADS, sz, c.stream>>>(g, tab, c.list, io);
+      CKR(launch_kernel(false, kz, persistent_grid(kz, SSFFT_THREADS, sz, itz, dev), SSFFT_THREADS, sz,
+                        c.stream, g, tab, c.list, io));
     }
     rec(1);
-    launch_y<T, TF, false, KRY>(p, g, c.cap, c.stream, tab, c.list);
+    CKR((launch_y<T, TF, false, KRY>(p, g, c.cap, c.stream, tab, c.list)));
     rec(2);
-    launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list);
+    CKR((launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list)));
     rec(3);
-    launch_y<T, TF, true, KRY>(p, g, c.cap, c.stream, tab, c.list);
+    CKR((launch_y<T, TF, true, KRY>(p, g, c.cap, c.stream, tab, c.list)));
     rec(4);
     if constexpr (PLANES) {
       if (dif_z) {
         auto k = dif_zinv_kernel<T>;
         const size_t sm = ((size_t)dz[1].p.elems + p.nz) * sizeof(cplx<T>);
         const int grid = persistent_grid(k, DIFZ_THREADS, sm, (long long)c.cap * 3 * dz[1].ntiles, dev);
-        launch_pdl(true, k, grid, DIFZ_THREADS, sm, c.stream, g, dz[1], tab, c.list, io, KRY ? 1 : 0);
+        CKR(launch_kernel(true, k, grid, DIFZ_THREADS, sm, c.stream, g, dz[1], tab, c.list, io, KRY ? 1 : 0));
       }
     }
     if (!dif_z) {
       auto kzi = zinv_kernel<T, TF, EPI>;
-      kzi<<<persistent_grid(kzi, SSFFT_THREADS, sz, itz, dev), SSFFT_THREADS, sz, c.stream>>>(g, tab, c.list, io);
+      CKR(launch_kernel(false, kzi, persistent_grid(kzi, SSFFT_THREADS, sz, itz, dev), SSFFT_THREADS, sz,
+                        c.stream, g, tab, c.list, io));
     }
     rec(5);
     if (c.launches) *c.launches += 5;
@@ -1335,21 +1201,19 @@ static int launch_krylov_iteration(const LaunchCtx &c, const SlotDev<T> *tab, bo
   const long long it = (long long)c.cap * vec_items(c.p->V);
   if (voxel) {
     auto k = krylov_update_kernel<T, PRO_TANGENT_VOXEL>;
-    launch_pdl(pdl_first, k, persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0,
-               c.stream, tab, c.list, c.p->V);
+    CKR(launch_kernel(pdl_first, k, persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0,
+                      c.stream, tab, c.list, c.p->V));
   } else {
     auto k = krylov_update_kernel<T, PRO_TANGENT_TABLE>;
-    launch_pdl(pdl_first, k, persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0,
-               c.stream, tab, c.list, c.p->V);
+    CKR(launch_kernel(pdl_first, k, persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0,
+                      c.stream, tab, c.list, c.p->V));
   }
   if (c.launches) *c.launches += 1;
-  CK(cudaGetLastError());
   CKR((launch_projector<T, T, PRO_TAU, EPI_PTAU>(c, tab, {}, ev)));
   auto ke = krylov_epilogue_kernel<T>;
-  launch_pdl(true, ke, persistent_grid(ke, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0, c.stream,
-             tab, c.list, c.p->V);
+  CKR(launch_kernel(true, ke, persistent_grid(ke, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0,
+                    c.stream, tab, c.list, c.p->V));
   if (c.launches) *c.launches += 1;
-  CK(cudaGetLastError());
   return 0;
 }
 
