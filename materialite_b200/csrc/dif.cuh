@@ -674,6 +674,9 @@ __device__ __forceinline__ void dif_y_middle(const DifTables<T, INV> &tb, const 
 // skips finished solves) or of the Newton correction, chosen at run time; or the residual's
 // Sbar - sigma.  What it writes: planes likewise, or the residual's or re-projection's epilogue.
 enum { DIF_PLANES = 0, DIF_RESIDUAL = 1, DIF_REPROJECT = 2 };
+constexpr int dif_kind(int epi) {
+  return epi == EPI_RESIDUAL ? DIF_RESIDUAL : (epi == EPI_REPROJECT ? DIF_REPROJECT : DIF_PLANES);
+}
 
 // tau of the component pair p at point v.
 template <typename T, typename TF, int KIND>

@@ -59,6 +59,8 @@ struct GridPlan {
   DifXPlan dx[2];
   DifXPlan dy[2];             // passes of planes too large for a block: y (tiles as the x pass's)
   DifZPlan dz[2][2];          // and z, forward and inverse
+  int cl_blocks[2], cl_threads[2];  // cluster passes: blocks a cluster (0: not used), their threads
+  int x_threads[2];           // threads of a Stockham x-pass block
   size_t partial_doubles;     // reduction partials per slot
 };
 
@@ -188,9 +190,8 @@ template <typename T> static int xpass_threads() {
 }
 
 template <typename T, typename TF, bool KRY>
-static int launch_xpass(const Grid<T> &g, size_t sx, long long items, int dev,
-                         cudaStream_t stream, const SlotDev<TF> *tab, SlotList list) {
-  const int pt = xpass_threads<T>();
+static int launch_xpass(const Grid<T> &g, int pt, size_t sx, long long items, int dev,
+                        cudaStream_t stream, const SlotDev<TF> *tab, SlotList list) {
   if constexpr (sizeof(T) == 4) {
     if (pt == 384) {
       auto k = xpass_kernel<T, TF, KRY, 384>;
@@ -204,11 +205,6 @@ static int launch_xpass(const Grid<T> &g, size_t sx, long long items, int dev,
   auto k = xpass_kernel<T, TF, KRY>;
   return launch_kernel(false, k, persistent_grid(k, XPASS_THREADS, sx, items, dev), XPASS_THREADS, sx,
                        stream, g, tab, list);
-}
-
-// The projection runs as three passes (z and y fused, in one block or one cluster).
-template <typename T> static bool three_pass(const GridPlan &p) {
-  return plane_ok<T>(p) || cluster_size<T>(p) > 0;
 }
 
 // Threads of a plane block: 1024 when a single block fits an SM (228 KB of shared memory),
@@ -394,7 +390,8 @@ static int launch_x(const GridPlan &p, const Grid<T> &g, long long cap, cudaStre
                      const SlotDev<TF> *tab, SlotList list) {
   const DifXPlan &P = p.dx[sizeof(T) == 8 ? 1 : 0];
   if (!P.ok)
-    return launch_xpass<T, TF, KRY>(g, smem_x_bytes<T>(g.kx, p.nx), cap * items_x(g), p.dev, stream, tab, list);
+    return launch_xpass<T, TF, KRY>(g, p.x_threads[sizeof(T) == 8 ? 1 : 0], smem_x_bytes<T>(g.kx, p.nx),
+                                    cap * items_x(g), p.dev, stream, tab, list);
   auto k = difx_of<T>(p.nx);
   const size_t sm = ((size_t)P.elems + p.nx) * sizeof(cplx<T>);
   const int grid = persistent_grid(k, DIFX_THREADS, sm, cap * P.nkx * p.ny, p.dev);
@@ -475,7 +472,33 @@ static void plan_free(GridPlan &p) {
     }
 }
 
-template <typename T, typename TF> static int set_kernel_attrs(const GridPlan &p, size_t smax);
+// The z and y passes of a projection: fused in one block (register-tiled or Stockham) or in a
+// cluster of C blocks, or passes of their own (z register-tiled where dif_z).
+enum { ROUTE_DIF_PLANE, ROUTE_CLUSTER, ROUTE_PLANE, ROUTE_LINES };
+struct Route {
+  int kind, C;
+  bool dif_z;
+};
+
+template <typename T, typename TF, int PRO, int EPI> static Route route_of(const GridPlan &p) {
+  const int k = sizeof(T) == 8 ? 1 : 0;
+  if (p.dplane[k][0].ok && p.dplane[k][1].ok) return {ROUTE_DIF_PLANE, 0, false};
+  // register-tiled z passes where nz has a plan and a pass only moves planes (the residual
+  // and the re-projection, one each a Newton iteration, keep the Stockham ones)
+  constexpr bool PLANES = sizeof(T) == sizeof(TF) && (PRO == PRO_INPUT || PRO == PRO_TAU) &&
+                          (EPI == EPI_STORE || EPI == EPI_PTAU);
+  const bool dif_z = PLANES && p.dz[k][0].ok && p.dz[k][1].ok;
+  // Five register-tiled passes beat three on clusters wherever both run (projections, us,
+  // clusters / five passes: 128^3 FP64 451 / 305, 64 x 128 x 144 FP64 280 / 190, 160^3 FP64
+  // 1203 / 615, 192^3 FP64 1725 / 1007 and float 830 / 580, 256^3 float 2201 / 1262).
+  if (!(dif_z && p.dy[k].ok)) {
+    if (p.cl_blocks[k]) return {ROUTE_CLUSTER, p.cl_blocks[k], false};
+    if (plane_ok<T>(p)) return {ROUTE_PLANE, 0, false};
+  }
+  return {ROUTE_LINES, 0, dif_z};
+}
+
+static int set_kernel_attrs(const GridPlan &p);
 
 static int plan_create(GridPlan &p, const ssfft_config *cfg, cudaStream_t stream) {
   memset(&p, 0, sizeof(p));
@@ -537,6 +560,12 @@ static int plan_create(GridPlan &p, const ssfft_config *cfg, cudaStream_t stream
       }
     }
   }
+  p.cl_blocks[0] = cluster_size<float>(p);
+  p.cl_blocks[1] = cluster_size<double>(p);
+  if (p.cl_blocks[0]) p.cl_threads[0] = cluster_threads<float>(p, p.cl_blocks[0]);
+  if (p.cl_blocks[1]) p.cl_threads[1] = cluster_threads<double>(p, p.cl_blocks[1]);
+  p.x_threads[0] = xpass_threads<float>();
+  p.x_threads[1] = xpass_threads<double>();
   // items of one slot per reduction, times the values each stores
   const Grid<double> &g = p.gd;
   size_t need = 0;
@@ -549,13 +578,7 @@ static int plan_create(GridPlan &p, const ssfft_config *cfg, cudaStream_t stream
       items_y(g) > (1 << 30) / 2)
     return ssfft_internal_fail(SSFFT_E_UNSUPPORTED, "grid too large for the reduction partials");
   p.partial_doubles = need;
-  if (p.fp64) {
-    CKR((set_kernel_attrs<double, double>(p, SMEM_LIMIT)));
-  } else {
-    CKR((set_kernel_attrs<float, float>(p, SMEM_LIMIT)));
-    CKR((set_kernel_attrs<double, float>(p, SMEM_LIMIT)));
-  }
-  return 0;
+  return set_kernel_attrs(p);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -566,96 +589,80 @@ template <typename F> static int smem_attr(F f, int m) {
   return 0;
 }
 
-template <typename T, typename TF, int PT> static int plane_attrs(int m) {
-  CKR(smem_attr(zyfwd_kernel<T, TF, PRO_INPUT, PT>, m));
-  CKR(smem_attr(zyfwd_kernel<T, TF, PRO_RESIDUAL, PT>, m));
-  CKR(smem_attr(zyfwd_kernel<T, TF, PRO_REPROJECT, PT>, m));
-  CKR(smem_attr(yzinv_kernel<T, TF, EPI_STORE, PT>, m));
-  CKR(smem_attr(yzinv_kernel<T, TF, EPI_RESIDUAL, PT>, m));
-  CKR(smem_attr(yzinv_kernel<T, TF, EPI_REPROJECT, PT>, m));
-  if (sizeof(T) == sizeof(TF)) {
-    CKR(smem_attr(zyfwd_kernel<T, T, PRO_TAU, PT>, m));
-    CKR(smem_attr(yzinv_kernel<T, T, EPI_PTAU, PT>, m));
-  }
-  return 0;
-}
-
-template <typename T, typename TF, int PT> static int cluster_attrs(int m) {
-  CKR(smem_attr(zyfwd_cl_kernel<T, TF, PRO_INPUT, PT>, m));
-  CKR(smem_attr(zyfwd_cl_kernel<T, TF, PRO_RESIDUAL, PT>, m));
-  CKR(smem_attr(zyfwd_cl_kernel<T, TF, PRO_REPROJECT, PT>, m));
-  CKR(smem_attr(yzinv_cl_kernel<T, TF, EPI_STORE, PT>, m));
-  CKR(smem_attr(yzinv_cl_kernel<T, TF, EPI_RESIDUAL, PT>, m));
-  CKR(smem_attr(yzinv_cl_kernel<T, TF, EPI_REPROJECT, PT>, m));
-  if (sizeof(T) == sizeof(TF)) {
-    CKR(smem_attr(zyfwd_cl_kernel<T, T, PRO_TAU, PT>, m));
-    CKR(smem_attr(yzinv_cl_kernel<T, T, EPI_PTAU, PT>, m));
-  }
-  return 0;
-}
-
-// The plane-pass instantiations of transforms in T with planes stored in TF.
-template <typename T, typename TF> static int dif_plane_attrs() {
-  const int m = DIF_SMEM_LIMIT;
-  CKR((smem_attr(dif_zyfwd_kernel<T, TF, DIF_PLANES>, m)));
-  if constexpr (sizeof(T) == sizeof(TF)) CKR((smem_attr(dif_yzinv_kernel<T, TF, DIF_PLANES>, m)));
-  if constexpr (sizeof(T) == 8) {
-    CKR((smem_attr(dif_zyfwd_kernel<double, double, DIF_RESIDUAL>, m)));
-    CKR((smem_attr(dif_yzinv_kernel<T, TF, DIF_RESIDUAL>, m)));
-    if constexpr (sizeof(TF) == 4) CKR((smem_attr(dif_yzinv_kernel<T, TF, DIF_REPROJECT>, m)));
-  }
-  return 0;
-}
-
-// Opt the shared-memory-hungry kernels of the plan's paths into up to `smax` bytes (the others
-// are not touched: the first touch of a kernel loads its code).
-template <typename T, typename TF> static int set_kernel_attrs(const GridPlan &p, size_t smax) {
-  const int m = (int)smax;
+// Opt the kernels of one projection into the shared memory they may ask for.  Nothing else is
+// named here: a kernel's first touch loads its code, and every kernel named is compiled.
+template <typename T, typename TF, int PRO, int EPI> static int projector_attrs(const GridPlan &p) {
+  const int m = (int)SMEM_LIMIT;
+  constexpr bool KRY = PRO_IS_KRYLOV(PRO) || PRO == PRO_TAU;
   const int k = sizeof(T) == 8 ? 1 : 0;
-  if constexpr (sizeof(T) == sizeof(TF)) CKR(smem_attr(constitutive_kernel<T>, (int)constitutive_smem_bytes()));
+  const Route r = route_of<T, TF, PRO, EPI>(p);
   if (p.dx[k].ok) {
     CKR(smem_attr(difx_of<T>(p.nx), m));
   } else {
-    CKR((smem_attr(xpass_kernel<T, TF, false>, m)));
-    CKR((smem_attr(xpass_kernel<T, TF, true>, m)));
+    const int pt = p.x_threads[k];
     if constexpr (sizeof(T) == 4) {
-      CKR((smem_attr(xpass_kernel<T, TF, false, 192>, m)));
-      CKR((smem_attr(xpass_kernel<T, TF, true, 192>, m)));
-      CKR((smem_attr(xpass_kernel<T, TF, false, 384>, m)));
-      CKR((smem_attr(xpass_kernel<T, TF, true, 384>, m)));
+      if (pt == 192) CKR((smem_attr(xpass_kernel<T, TF, KRY, 192>, m)));
+      if (pt == 384) CKR((smem_attr(xpass_kernel<T, TF, KRY, 384>, m)));
     }
+    if (pt == XPASS_THREADS) CKR((smem_attr(xpass_kernel<T, TF, KRY>, m)));
   }
-  if (p.dplane[k][0].ok && p.dplane[k][1].ok) return dif_plane_attrs<T, TF>();
+  if (r.kind == ROUTE_DIF_PLANE) {
+    if constexpr (PRO == PRO_RESIDUAL)
+      CKR((smem_attr(dif_zyfwd_kernel<double, double, DIF_RESIDUAL>, DIF_SMEM_LIMIT)));
+    else
+      CKR((smem_attr(dif_zyfwd_kernel<T, TF, DIF_PLANES>, DIF_SMEM_LIMIT)));
+    return smem_attr(dif_yzinv_kernel<T, TF, dif_kind(EPI)>, DIF_SMEM_LIMIT);
+  }
+  if (r.kind == ROUTE_CLUSTER) {
+    const int pt = p.cl_threads[k];
+    if (pt == 1024) {
+      CKR((smem_attr(zyfwd_cl_kernel<T, TF, PRO, 1024>, m)));
+      return smem_attr(yzinv_cl_kernel<T, TF, EPI, 1024>, m);
+    }
+    if (pt == 256) {
+      CKR((smem_attr(zyfwd_cl_kernel<T, TF, PRO, 256>, m)));
+      return smem_attr(yzinv_cl_kernel<T, TF, EPI, 256>, m);
+    }
+    CKR((smem_attr(zyfwd_cl_kernel<T, TF, PRO, 512>, m)));
+    return smem_attr(yzinv_cl_kernel<T, TF, EPI, 512>, m);
+  }
+  if (r.kind == ROUTE_PLANE) {
+    if (plane_threads<T>(p) == 1024) {
+      CKR((smem_attr(zyfwd_kernel<T, TF, PRO, 1024>, m)));
+      return smem_attr(yzinv_kernel<T, TF, EPI, 1024>, m);
+    }
+    CKR((smem_attr(zyfwd_kernel<T, TF, PRO, 512>, m)));
+    return smem_attr(yzinv_kernel<T, TF, EPI, 512>, m);
+  }
   if (p.dy[k].ok) {
     CKR((smem_attr(dify_kernel<T, false>, m)));
     CKR((smem_attr(dify_kernel<T, true>, m)));
+  } else {
+    CKR((smem_attr(ypass_kernel<T, TF, false, KRY>, m)));
+    CKR((smem_attr(ypass_kernel<T, TF, true, KRY>, m)));
   }
   if constexpr (sizeof(T) == sizeof(TF)) {
-    if (p.dz[k][0].ok && p.dz[k][1].ok) {
+    if (r.dif_z) {
       CKR(smem_attr(dif_zfwd_kernel<T>, m));
-      CKR(smem_attr(dif_zinv_kernel<T>, m));
+      return smem_attr(dif_zinv_kernel<T>, m);
     }
   }
-  CKR(smem_attr(zfwd_kernel<T, TF, PRO_INPUT>, m));
-  CKR(smem_attr(zfwd_kernel<T, TF, PRO_RESIDUAL>, m));
-  CKR(smem_attr(zfwd_kernel<T, TF, PRO_REPROJECT>, m));
-  CKR((smem_attr(ypass_kernel<T, TF, false, false>, m)));
-  CKR((smem_attr(ypass_kernel<T, TF, true, false>, m)));
-  CKR((smem_attr(ypass_kernel<T, TF, false, true>, m)));
-  CKR((smem_attr(ypass_kernel<T, TF, true, true>, m)));
-  CKR(smem_attr(zinv_kernel<T, TF, EPI_STORE>, m));
-  CKR(smem_attr(zinv_kernel<T, TF, EPI_RESIDUAL>, m));
-  CKR(smem_attr(zinv_kernel<T, TF, EPI_REPROJECT>, m));
-  CKR((plane_attrs<T, TF, 512>(m)));
-  CKR((plane_attrs<T, TF, 1024>(m)));
-  CKR((cluster_attrs<T, TF, 256>(m)));
-  CKR((cluster_attrs<T, TF, 512>(m)));
-  CKR((cluster_attrs<T, TF, 1024>(m)));
-  if (sizeof(T) == sizeof(TF)) {
-    CKR(smem_attr(zfwd_kernel<T, T, PRO_TAU>, m));
-    CKR(smem_attr(zinv_kernel<T, T, EPI_PTAU>, m));
-  }
+  CKR(smem_attr(zfwd_kernel<T, TF, PRO>, m));
+  return smem_attr(zinv_kernel<T, TF, EPI>, m);
+}
+
+// The projections of a plan: of a given field, of a Krylov iteration, of the residual, and in
+// mixed precision of the Newton correction.
+template <typename T> static int solve_attrs(const GridPlan &p) {
+  CKR(smem_attr(constitutive_kernel<T>, (int)constitutive_smem_bytes()));
+  CKR((projector_attrs<T, T, PRO_INPUT, EPI_STORE>(p)));
+  CKR((projector_attrs<T, T, PRO_TAU, EPI_PTAU>(p)));
+  CKR((projector_attrs<double, T, PRO_RESIDUAL, EPI_RESIDUAL>(p)));
+  if constexpr (sizeof(T) == 4) CKR((projector_attrs<double, T, PRO_REPROJECT, EPI_REPROJECT>(p)));
   return 0;
+}
+static int set_kernel_attrs(const GridPlan &p) {
+  return p.fp64 ? solve_attrs<double>(p) : solve_attrs<float>(p);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1037,10 +1044,10 @@ struct LaunchCtx {
 // The register-tiled plane passes of one projection around the x pass.
 template <typename T, typename TF, int PRO, int EPI, typename REC>
 static int launch_dif_planes(const LaunchCtx &c, const SlotDev<TF> *tab, const ExtIO<TF> &io,
-                              const DifPlane *PP, const REC &rec) {
-  const DifPlane &P = PP[0], &Q = PP[1];
+                              const REC &rec) {
   constexpr bool KRY = PRO == PRO_TAU;
   const GridPlan &p = *c.p;
+  const DifPlane *PP = p.dplane[sizeof(T) == 8 ? 1 : 0], &P = PP[0], &Q = PP[1];
   const Grid<T> &g = grid_of<T>(p);
   const size_t sp = DifTables<T, false>::bytes(P, p.ny, p.nz, g.hs);
   const size_t sq = DifTables<T, true>::bytes(Q, p.ny, p.nz, g.hs);
@@ -1061,8 +1068,7 @@ static int launch_dif_planes(const LaunchCtx &c, const SlotDev<TF> *tab, const E
   CKR((launch_x<T, TF, KRY>(p, g, c.cap, c.stream, tab, c.list)));
   rec(3);
   rec(4);
-  constexpr int KIND = EPI == EPI_RESIDUAL ? DIF_RESIDUAL : (EPI == EPI_REPROJECT ? DIF_REPROJECT : DIF_PLANES);
-  auto ki = dif_yzinv_kernel<T, TF, KIND>;
+  auto ki = dif_yzinv_kernel<T, TF, dif_kind(EPI)>;
   return launch_kernel(true, ki, persistent_grid(ki, pt, sq, it, p.dev), pt, sq, c.stream, g, Q, tab,
                        c.list, io, (int)EPI);
 }
@@ -1082,27 +1088,18 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
     if (ev) cudaEventRecord(ev[k], c.stream);
   };
   const int dev = p.dev;
-  const DifPlane *dp = p.dplane[sizeof(T) == 8 ? 1 : 0];
-  // register-tiled z passes where nz has a plan and a pass only moves planes (the residual
-  // and the re-projection, one each a Newton iteration, keep the Stockham ones)
-  const DifZPlan *dz = p.dz[sizeof(T) == 8 ? 1 : 0];
-  constexpr bool PLANES = sizeof(T) == sizeof(TF) && (PRO == PRO_INPUT || PRO == PRO_TAU) &&
-                          (EPI == EPI_STORE || EPI == EPI_PTAU);
-  const bool dif_z = PLANES && dz[0].ok && dz[1].ok;
-  // Five register-tiled passes beat three on clusters wherever both run (projections, us,
-  // clusters / five passes: 128^3 FP64 451 / 305, 64 x 128 x 144 FP64 280 / 190, 160^3 FP64
-  // 1203 / 615, 192^3 FP64 1725 / 1007 and float 830 / 580, 256^3 float 2201 / 1262).
-  const bool five = dif_z && p.dy[sizeof(T) == 8 ? 1 : 0].ok;
+  const Route r = route_of<T, TF, PRO, EPI>(p);
   rec(0);
-  if (dp[0].ok && dp[1].ok) {
-    CKR((launch_dif_planes<T, TF, PRO, EPI>(c, tab, io, dp, rec)));
+  if (r.kind == ROUTE_DIF_PLANE) {
+    CKR((launch_dif_planes<T, TF, PRO, EPI>(c, tab, io, rec)));
     rec(5);
     if (c.launches) *c.launches += 3;
-  } else if (const int C = five ? 0 : cluster_size<T>(p)) {
+  } else if (r.kind == ROUTE_CLUSTER) {
+    const int C = r.C;
     const ClusterGeo q = cluster_geo<T>(p, C);
     const size_t sp = smem_cplane_bytes<T>(p.ny, p.nz, g.hs, C);
     const long long it = (long long)c.cap * items_plane(g);
-    const int pt = cluster_threads<T>(p, C);
+    const int pt = p.cl_threads[sizeof(T) == 8 ? 1 : 0];
     if (pt == 1024)
       CKR(launch_clustered(zyfwd_cl_kernel<T, TF, PRO, 1024>, C, 1024, sp, it, dev, c.stream, g, q, tab, c.list, io));
     else if (pt == 256)
@@ -1122,7 +1119,7 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
       CKR(launch_clustered(yzinv_cl_kernel<T, TF, EPI, 512>, C, 512, sp, it, dev, c.stream, g, q, tab, c.list, io));
     rec(5);
     if (c.launches) *c.launches += 3;
-  } else if (plane_ok<T>(p)) {
+  } else if (r.kind == ROUTE_PLANE) {
     const size_t sp = smem_plane_bytes<T>(p.ny, p.nz);
     const long long it = (long long)c.cap * items_plane(g);
     if (plane_threads<T>(p) == 1024) {
@@ -1149,15 +1146,16 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
   } else {
     const size_t sz = smem_z_bytes<T>(p.lz, p.nz);
     const long long itz = (long long)c.cap * items_z(g);
-    if constexpr (PLANES) {
-      if (dif_z) {
+    const DifZPlan *dz = p.dz[sizeof(T) == 8 ? 1 : 0];
+    if constexpr (sizeof(T) == sizeof(TF)) {
+      if (r.dif_z) {
         auto k = dif_zfwd_kernel<T>;
         const size_t sm = ((size_t)dz[0].p.elems + p.nz) * sizeof(cplx<T>);
         const int grid = persistent_grid(k, DIFZ_THREADS, sm, (long long)c.cap * 3 * dz[0].ntiles, dev);
         CKR(launch_kernel(KRY, k, grid, DIFZ_THREADS, sm, c.stream, g, dz[0], tab, c.list, io, KRY ? 1 : 0));
       }
     }
-    if (!dif_z) {
+    if (!r.dif_z) {
       auto kz = zfwd_kernel<T, TF, PRO>;
       CKR(launch_kernel(false, kz, persistent_grid(kz, SSFFT_THREADS, sz, itz, dev), SSFFT_THREADS, sz,
                         c.stream, g, tab, c.list, io));
@@ -1169,15 +1167,15 @@ static int launch_projector(const LaunchCtx &c, const SlotDev<TF> *tab, ExtIO<TF
     rec(3);
     CKR((launch_y<T, TF, true, KRY>(p, g, c.cap, c.stream, tab, c.list)));
     rec(4);
-    if constexpr (PLANES) {
-      if (dif_z) {
+    if constexpr (sizeof(T) == sizeof(TF)) {
+      if (r.dif_z) {
         auto k = dif_zinv_kernel<T>;
         const size_t sm = ((size_t)dz[1].p.elems + p.nz) * sizeof(cplx<T>);
         const int grid = persistent_grid(k, DIFZ_THREADS, sm, (long long)c.cap * 3 * dz[1].ntiles, dev);
         CKR(launch_kernel(true, k, grid, DIFZ_THREADS, sm, c.stream, g, dz[1], tab, c.list, io, KRY ? 1 : 0));
       }
     }
-    if (!dif_z) {
+    if (!r.dif_z) {
       auto kzi = zinv_kernel<T, TF, EPI>;
       CKR(launch_kernel(false, kzi, persistent_grid(kzi, SSFFT_THREADS, sz, itz, dev), SSFFT_THREADS, sz,
                         c.stream, g, tab, c.list, io));
