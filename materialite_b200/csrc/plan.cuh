@@ -59,6 +59,7 @@ struct GridPlan {
   DifXPlan dx[2];
   DifXPlan dy[2];             // passes of planes too large for a block: y (tiles as the x pass's)
   DifZPlan dz[2][2];          // and z, forward and inverse
+  bool few[2];                // given fields' projections in clusters although one block would do
   int cl_blocks[2], cl_threads[2];  // cluster passes: blocks a cluster (0: not used), their threads
   int x_threads[2];           // threads of a Stockham x-pass block
   size_t partial_doubles;     // reduction partials per slot
@@ -374,6 +375,47 @@ template <typename T> static DifZPlan dif_zplan(long long lines, int nz, bool in
   return P;
 }
 
+// Sum of the factors 5 and 7 of a length, which the Stockham passes transform by direct sums.
+static int direct_sum_weight(int n) {
+  int w = 0;
+  for (int f : {5, 7})
+    for (; n % f == 0; n /= f) w += f;
+  return w;
+}
+
+// Small long planes keep the Stockham passes where the register-tiled ones have a plan too: a
+// register-tiled block has a thread for eight points, and its chain of stages along a long axis
+// is longer.  Projections in us, register-tiled / Stockham: 8 x 1 x 512 FP64 37.9 / 30.5,
+// 8 x 512 x 1 39.0 / 33.5, 64 x 8 x 64 36.7 / 32.8, 8 x 8 x 256 mixed 35.0 / 32.6; Krylov
+// iterations 5 to 20% faster.  Near-square planes of as many points lose or draw (30 x 20 1.2
+// times slower), as do planes of twice the points (8 x 8 x 512 FP64 42.3 / 51.2), axes with direct
+// sums, and grids of more than about 1024 points an SM in double and 2048 in float (128 x 8 x 128
+// FP64 42.7 / 48.9, 160 x 16 x 128 mixed 50.6 / 53.9).  The rule follows from the grid alone, so
+// a solve's arithmetic does not depend on its batch.
+template <typename T> static bool long_plane(const GridPlan &p) {
+  const bool pow2 = (p.ny & (p.ny - 1)) == 0 && (p.nz & (p.nz - 1)) == 0;
+  const bool lng = p.nz >= (pow2 ? 4 : 8) * p.ny || p.ny >= 128 * p.nz;
+  const int pts = p.ny * p.nz, most = sizeof(T) == 4 ? 2048 : 1024;
+  return lng && direct_sum_weight(p.ny) + direct_sum_weight(p.nz) == 0 && pts <= most &&
+         3LL * p.nx * pts <= 148LL * most;
+}
+
+// Projections of a given field on grids of few planes, each of 96 KB and more in float or of the
+// size that clusters of four split in double: one block an SM leaves most of the chip idle where
+// a cluster takes four SMs a plane.  In us, one block / cluster: 8 x 144 x 144 mixed 65.5 / 50.4,
+// 8 x 128 x 128 mixed 53 / 47, 8 x 384 x 32 FP64 73.4 / 55.0, 8 x 640 x 20 FP64 80 / 74.  With
+// direct sums the clusters lose (8 x 100 x 100 FP64 62 / 71, 6 x 160 x 160 mixed 72 / 76), and
+// past 33 of them they share SMs (12 x 640 x 20 FP64 82 / 113, 24 x 144 x 144 mixed 71 / 84).
+// Krylov iterations stay in one block: a group runs them for many slots at once, and a solve's
+// arithmetic must not depend on its batch.
+template <typename T> static bool few_planes(const GridPlan &p) {
+  if (3 * p.nx > 33) return false;
+  const int w = direct_sum_weight(p.ny) + direct_sum_weight(p.nz), C = cluster_size<T>(p);
+  if (sizeof(T) == 8) return w <= 10 && C >= 4;
+  return w == 0 && p.ny * p.nz >= 12288 &&
+         (C ? smem_cplane_bytes<T>(p.ny, p.nz, p.gd.hs, C) <= 113 * 1024 : plane_ok<T>(p));
+}
+
 // The register-tiled x pass of lines of nx points.
 template <typename T>
 static void (*difx_of(int nx))(Grid<T>, DifXPlan, const SlotDev<T> *, SlotList, int) {
@@ -482,7 +524,8 @@ struct Route {
 
 template <typename T, typename TF, int PRO, int EPI> static Route route_of(const GridPlan &p) {
   const int k = sizeof(T) == 8 ? 1 : 0;
-  if (p.dplane[k][0].ok && p.dplane[k][1].ok) return {ROUTE_DIF_PLANE, 0, false};
+  const bool few = PRO == PRO_INPUT && p.few[k];
+  if (p.dplane[k][0].ok && p.dplane[k][1].ok && !few) return {ROUTE_DIF_PLANE, 0, false};
   // register-tiled z passes where nz has a plan and a pass only moves planes (the residual
   // and the re-projection, one each a Newton iteration, keep the Stockham ones)
   constexpr bool PLANES = sizeof(T) == sizeof(TF) && (PRO == PRO_INPUT || PRO == PRO_TAU) &&
@@ -491,7 +534,7 @@ template <typename T, typename TF, int PRO, int EPI> static Route route_of(const
   // Five register-tiled passes beat three on clusters wherever both run (projections, us,
   // clusters / five passes: 128^3 FP64 451 / 305, 64 x 128 x 144 FP64 280 / 190, 160^3 FP64
   // 1203 / 615, 192^3 FP64 1725 / 1007 and float 830 / 580, 256^3 float 2201 / 1262).
-  if (!(dif_z && p.dy[k].ok)) {
+  if (!(dif_z && p.dy[k].ok) || few) {
     if (p.cl_blocks[k]) return {ROUTE_CLUSTER, p.cl_blocks[k], false};
     if (plane_ok<T>(p)) return {ROUTE_PLANE, 0, false};
   }
@@ -548,9 +591,14 @@ static int plan_create(GridPlan &p, const ssfft_config *cfg, cudaStream_t stream
     }
   }
   if (p.ny * p.nz >= DIF_MIN_PLANE && env_int("SSFFT_XPASS_KX") <= 0 && env_int("SSFFT_XPASS_THREADS") <= 0) {
-    p.dx[0] = dif_xplan<float>(p.nx, p.ny, p.gd.hs);
-    p.dx[1] = dif_xplan<double>(p.nx, p.ny, p.gd.hs);
-    // SSFFT_NO_PLANE keeps the Stockham five-pass kernels, SSFFT_CLUSTER the cluster passes
+    // two kinds of grid are short of work in the tiles and keep the Stockham pass: a single
+    // column on long lines without direct sums in float, whose tiles are four wide (768 x 768 x 1:
+    // the projection takes 289 us, 198 there; 800 x 800 x 1 227 and 287; at 48 points along x
+    // up to 10% more there), and in double "lines" of one point, which fill 24 of 192 threads
+    // (1 x 512 x 512: 170 us, 119)
+    if (p.gd.hs > 1 || p.nx < 256 || direct_sum_weight(p.nx)) p.dx[0] = dif_xplan<float>(p.nx, p.ny, p.gd.hs);
+    if (p.nx > 1) p.dx[1] = dif_xplan<double>(p.nx, p.ny, p.gd.hs);
+    // SSFFT_NO_PLANE and SSFFT_CLUSTER choose among the Stockham z and y passes
     if (p.use_plane && env_int("SSFFT_CLUSTER") <= 0) {
       p.dy[0] = dif_yplan<float>(p.nx, p.ny, p.gd.hs);
       p.dy[1] = dif_yplan<double>(p.nx, p.ny, p.gd.hs);
@@ -559,6 +607,12 @@ static int plan_create(GridPlan &p, const ssfft_config *cfg, cudaStream_t stream
         p.dz[1][d] = dif_zplan<double>((long long)p.nx * p.ny, p.nz, d == 1);
       }
     }
+  }
+  for (int k = 0; k < 2; ++k) {
+    if (!p.dplane[k][0].ok || !p.dplane[k][1].ok) continue;
+    p.few[k] = k ? few_planes<double>(p) : few_planes<float>(p);
+    if (k ? long_plane<double>(p) : long_plane<float>(p))
+      p.dplane[k][0].ok = p.dy[k].ok = p.dz[k][0].ok = 0;
   }
   p.cl_blocks[0] = cluster_size<float>(p);
   p.cl_blocks[1] = cluster_size<double>(p);
