@@ -68,10 +68,10 @@ WORKLOADS = {
 }
 
 def plane_path(n):
-    """True when the z and y passes of an n^3 float solve run plane-fused: in one block (a
-    padded yz plane pair of complex floats fits the 200 KB shared-memory budget) or split
-    over a thread-block cluster of 2, 4 or 8 blocks, each holding two buffers of its rows'
-    padded z lines (or of its columns' y lines) within the same budget."""
+    """True when the Stockham z and y passes of an n^3 float solve can run plane-fused: in one
+    block (a padded yz plane pair of complex floats fits the 200 KB shared-memory budget) or
+    split over a thread-block cluster of 2, 4 or 8 blocks, each holding two buffers of its
+    rows' padded z lines (or of its columns' y lines) within the same budget."""
     padded = lambda m: m + (m >> 4) + 1
     if (2 * padded(n * (n + 2)) + 2 * n) * 8 <= 200 * 1024:
         return True
@@ -85,6 +85,18 @@ def plane_path(n):
     return False
 
 
+def separate_y_passes(n):
+    """True when the Krylov iterations of an n^3 float solve transform y in passes of their
+    own.  Lengths with prime factors up to 7 have register-tiled passes: one block holds a
+    plane in place up to 160 points an axis (224 KB with its padding), five passes take
+    larger ones.  Other lengths run the Stockham passes."""
+    m = n
+    for f in (2, 3, 5, 7):
+        while m % f == 0:
+            m //= f
+    return n > 160 if m == 1 else not plane_path(n)
+
+
 # Algorithmic HBM bytes per voxel of each Krylov-iteration kernel with float fields:
 # planar vectors are 24 B/voxel (6 x 4 B); the stored half spectrum is 6 x hs/n x 8 B with
 # hs = n/2 columns on even grids (the zeroed Nyquist column is not stored), (n+1)/2 on odd.
@@ -92,11 +104,12 @@ def plane_path(n):
 # writes u', w, x) and writes tau = K v over y'; the forward z pass reads tau and writes the
 # spectrum; the inverse z pass writes P tau over y', which the epilogue kernel turns into
 # y' (with the MINRES dot products).  With the plane-fused passes the y transforms happen in
-# shared memory inside the z kernels and move no bytes of their own.
-def kernel_bytes_per_voxel(n, table_mode=True):
+# shared memory inside the z kernels and move no bytes of their own (y_passes: whether the
+# iteration has y passes of its own; None: by the rule above).
+def kernel_bytes_per_voxel(n, table_mode=True, y_passes=None):
     spec = 6 * (n // 2 if n % 2 == 0 else n // 2 + 1) / n * 8.0
     kin = 4.0 if table_mode else 84.0
-    ypass = 0.0 if plane_path(n) else 2 * spec
+    ypass = 2 * spec if (separate_y_passes(n) if y_passes is None else y_passes) else 0.0
     return {
         "zfwd": 24.0 + spec,                # read tau; write spectrum
         "yfwd": ypass,
@@ -713,6 +726,15 @@ def request_mode(args, w):
           flush=True)
 
 
+def kernels_per_iteration(h):
+    """Kernels of one Krylov iteration of a solved handle, from its launch counter."""
+    counts = [h.stats()[1]]
+    for reps in (1, 2):
+        h.profile_krylov(reps=reps)
+        counts.append(h.stats()[1])
+    return (counts[2] - counts[1]) - (counts[1] - counts[0])
+
+
 def kernels_mode(args, w):
     """One load increment of the workload, then the Krylov-iteration kernels timed with
     CUDA events on the handle's stream (``--reps`` iterations); prints microseconds and
@@ -720,12 +742,13 @@ def kernels_mode(args, w):
     rot, ids = build_microstructure(w)
     h = make_handle(w, rot, ids, 0)
     run_solve(h, dict(w, steps=1))
+    kernels = kernels_per_iteration(h)
     prof = h.profile_krylov(reps=args.reps)
     h.close()
     n = w["n"]
     V = n ** 3
-    bpv = kernel_bytes_per_voxel(n, table_mode=w.get("model") != "evp")
-    out = {"workload": args.workload, "plane_path": plane_path(n), "reps": args.reps,
+    bpv = kernel_bytes_per_voxel(n, table_mode=w.get("model") != "evp", y_passes=kernels == 7)
+    out = {"workload": args.workload, "kernels_per_iteration": kernels, "reps": args.reps,
            "iteration_us": prof[7] * 1e6,
            "iteration_gbs": sum(bpv.values()) * V / prof[7] / 1e9, "kernels": {}}
     for i, k in enumerate(KERNEL_NAMES):
