@@ -798,12 +798,11 @@ def accuracy_mode(args, w):
 
 
 # DRAM read + write bytes of one steady-state launch of each Krylov kernel on plain128
-# (128^3, mixed precision; the transforms as cluster passes), from one-launch ncu captures of
-# `--mode kernels --workload plain128` (profiles/krylov_kernels_plain128.md).  The update
-# kernel reads 260.1 MB and writes 154.2 MB against 461 MB algorithmic: part of its writes
-# are still in L2 when it ends.
-PLAIN128_TRAFFIC_BYTES = {"update": 414.4e6, "epilogue": 171.7e6, "zfwd": 57.1e6,
-                          "xpass": 52.6e6, "zinv": 58.7e6}
+# (128^3, mixed precision), from one-launch ncu captures of `--mode kernels --workload plain128`
+# (profiles/krylov_kernels_plain128.md).  The update kernel reads 260.1 MB and writes 153.4 MB
+# against 461 MB algorithmic: part of its writes are still in L2 when it ends.
+PLAIN128_TRAFFIC_BYTES = {"update": 413.6e6, "epilogue": 167.7e6, "zfwd": 57.6e6,
+                          "xpass": 50.6e6, "zinv": 60.0e6}
 
 
 def plain128_roofline(device):
