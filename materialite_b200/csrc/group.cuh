@@ -454,7 +454,7 @@ struct Group {
     else
       CKR(launch_reproject_update<T>(lctx(GL_TAIL, s), tab));
     CKR(launch_constitutive<T>(lctx(GL_NEWTON, s), tab, false));
-    group_swap_stress_kernel<T><<<1, 32, 0, s>>>(tab, dids, dcounts, B);
+    CKR(launch_kernel(false, group_swap_stress_kernel<T>, 1, 32, 0, s, tab, dids, dcounts, B));
     ++launches;
     CKR(launch_residual<T>(lctx(GL_NEWTON, s), tab));
     CKR(launch_norms<T>(lctx(GL_NEWTON, s), tab));

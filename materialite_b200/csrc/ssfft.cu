@@ -157,8 +157,9 @@ template <typename T> static int run_minres(ssfft_handle *h, long long *iters) {
         cudaGraphDestroy(graph);
         return fail(SSFFT_E_CUDA, std::string("device loop setup: ") + cudaGetErrorString(e));
       }
-      const int rc = chunk();
-      minres_continue_kernel<<<1, 32, 0, h->stream>>>(h->sb.st, cond);
+      int rc = chunk();
+      // without this kernel the loop would never end
+      if (!rc) rc = launch_kernel(false, minres_continue_kernel, 1, 32, 0, h->stream, h->sb.st, cond);
       cudaGraph_t captured = nullptr;
       e = cudaStreamEndCapture(h->stream, &captured);
       h->chunk_kernels = (int)(h->launches - launches_before);
@@ -877,15 +878,20 @@ extern "C" int ssfft_apply_projection(ssfft_handle *h, const double *in_host, do
                                   cudaMemcpyHostToDevice, h->stream);
   if (e == cudaSuccess) {
     if (h->plan.fp64) {
-      from_point_major_kernel<double><<<eb, SSFFT_THREADS, 0, h->stream>>>(V, tmp, (double *)a);
-      rc = apply_projection_dev<double>(h, (const double *)a, (double *)bb);
-      to_point_major_kernel<double><<<eb, SSFFT_THREADS, 0, h->stream>>>(V, 6, (const double *)bb, tmp);
+      rc = launch_kernel(false, from_point_major_kernel<double>, eb, SSFFT_THREADS, 0, h->stream, V, tmp,
+                         (double *)a);
+      if (!rc) rc = apply_projection_dev<double>(h, (const double *)a, (double *)bb);
+      if (!rc)
+        rc = launch_kernel(false, to_point_major_kernel<double>, eb, SSFFT_THREADS, 0, h->stream, V, 6,
+                           (const double *)bb, tmp);
     } else {
-      from_point_major_kernel<float><<<eb, SSFFT_THREADS, 0, h->stream>>>(V, tmp, (float *)a);
-      rc = apply_projection_dev<float>(h, (const float *)a, (float *)bb);
-      to_point_major_kernel<float><<<eb, SSFFT_THREADS, 0, h->stream>>>(V, 6, (const float *)bb, tmp);
+      rc = launch_kernel(false, from_point_major_kernel<float>, eb, SSFFT_THREADS, 0, h->stream, V, tmp,
+                         (float *)a);
+      if (!rc) rc = apply_projection_dev<float>(h, (const float *)a, (float *)bb);
+      if (!rc)
+        rc = launch_kernel(false, to_point_major_kernel<float>, eb, SSFFT_THREADS, 0, h->stream, V, 6,
+                           (const float *)bb, tmp);
     }
-    e = cudaGetLastError();
   }
   if (e == cudaSuccess && rc == 0)
     e = cudaMemcpyAsync(out_host, tmp, (size_t)V * 6 * sizeof(double), cudaMemcpyDeviceToHost,
