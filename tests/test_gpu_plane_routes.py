@@ -5,6 +5,9 @@
   the five register-tiled passes in float (192 x 192: 307 KB in one block).
 * The planes that come closest to the 229,376 bytes one block may take: 224 x 125 (229,284) and
   175 x 160 (228,750) in float, 140 x 98 (226,044) in double.
+* An elastic solve on register-tiled passes against one on Stockham passes throughout, x included
+  (SSFFT_XPASS_THREADS takes the Stockham x pass): both meet a residual of 1e-10 (FP64) or 1e-6
+  of the stress, so their stresses may differ by that times the grains' stiffness contrast.
 * Three slots of one group in five register-tiled passes, the second with a quarter of the load
   steps, so that its solves are over while its neighbours' go on, against the solver handle.
 
@@ -73,3 +76,29 @@ def test_group_of_five_pass_solves(dims, precision):
             assert np.array_equal(h.field("stress"), r.stress)
         finally:
             h.close()
+
+
+@pytest.mark.parametrize("dims,precision,gtol", [((3, 135, 125), "fp64", 1e-10),
+                                                 ((24, 20, 27), "fp64", 1e-10),
+                                                 ((2, 192, 175), "mixed", 1e-6),
+                                                 ((20, 45, 40), "mixed", 1e-6)])
+def test_solve_as_on_stockham_passes_throughout(monkeypatch, dims, precision, gtol):
+    from materialite_b200.microstructure import bunge_random_rotations, periodic_voronoi
+    rng = np.random.default_rng(5)
+    grain = periodic_voronoi(dims, 6, rng).astype(np.int32)
+    rotations = bunge_random_rotations(6, rng)
+    stress = []
+    for stockham in (False, True):
+        if stockham:
+            monkeypatch.setenv("SSFFT_NO_PLANE", "1")
+            monkeypatch.setenv("SSFFT_XPASS_THREADS", "192")
+        h = SolverHandle(dims, MASK, precision, global_tolerance=gtol,
+                         linear_solver_tolerance=0.01 * gtol)
+        try:
+            h.set_phases([PhaseSpec("elastic", C_CUBIC)])
+            h.set_microstructure(rotations, grain)
+            h.solve_constant_rates(np.array([1e-3, 0, 0, 0, 0, 0]), np.zeros(6), 1.0, 1.0)
+            stress.append(h.field("stress"))
+        finally:
+            h.close()
+    assert np.linalg.norm(stress[0] - stress[1]) <= 4 * gtol * np.linalg.norm(stress[1])
