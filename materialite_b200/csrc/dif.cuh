@@ -244,9 +244,9 @@ struct DifXPlan {
   FastDiv fd_mid, fd_r2, fd_items, fd_nkx;
 };
 
-// MB blocks an SM: five in float.  In double three (96 registers), which hide more of the
-// latency than two (168), up to 200 points along x, and two for longer lines, whose tiles of
-// 46 KB and more are in flight enough at two blocks and whose radix-16 stages spill at three.
+// MB blocks an SM: five in float.  In double three (96 registers, 32 bytes spilled), which hide
+// more of the latency than two (168), up to 200 points along x, and two for longer lines, whose
+// tiles take 46 KB and more.  Both run the same stages; the line is where the sweep crosses.
 // Projections in FP64, us, two / three blocks: 45 x 50 x 63 47.3 / 44.7, 96 x 80 x 60 82.0 / 76.8,
 // 135 x 175 x 189 771 / 723, 128^3 305 / 297, 192^3 1007 / 1008, 200 x 225 x 64 469 / 460;
 // 240 x 96 x 250 977 / 1051, 256^3 2177 / 2320.

@@ -61,7 +61,8 @@ def unique_rotations(R):
     R = np.ascontiguousarray(np.asarray(R, dtype=np.float64).reshape(-1, 9))
     # points share their grain's rotation: equal bit patterns are found by sorting one 64-bit
     # hash a point (checked against the rows), and only the distinct rows are sorted by value.
-    # np.unique over the rows takes 45 ms of a 32^3 drop-in call, this 4 ms.
+    # At 32^3 and 60 grains np.unique over the rows takes 104 ms, this 5 ms; with too many
+    # grains for the sample to show repeats (700 at 100^3) every row is sorted, as there.
     rows, point = R, None
     bits = R.view(np.uint64)
     key = bits @ _ROW_HASH
