@@ -185,6 +185,37 @@ __device__ __forceinline__ double block_max(double v, double *scratch) {
   return v;
 }
 
+// The sum that block_sum forms from the sums of its first W warps (of eight), in its order.
+__device__ __forceinline__ double warps_sum(const double *w, int W = 8) {
+  double v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = (i < W ? w[i] : 0.0) + 0.0;
+  return ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
+}
+
+// Reduce N = 16 or 32 values over a warp by halving: a lane passes on half of its values in each
+// step and keeps the others, so N - 1 shuffles (and one more for 16) do the work of 5 N.  Each
+// value is combined in the order of warp_sum.  Lane l then holds value warp_value<N>(l).
+template <int N, typename OP> __device__ __forceinline__ double warp_reduce_many(double *a, OP op) {
+  const int lane = threadIdx.x & 31;
+  int base = 0;
+#pragma unroll
+  for (int h = N / 2, o = 16; h > 0; h /= 2, o /= 2) {
+    const bool up = lane & o;
+    if (up) base += h;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const double keep = up ? a[i + h] : a[i], give = up ? a[i] : a[i + h];
+      a[i] = op(base + i, keep, __shfl_xor_sync(0xffffffffu, give, o));
+    }
+  }
+  if (N == 16) a[0] = op(base, a[0], __shfl_xor_sync(0xffffffffu, a[0], 1));
+  return a[0];
+}
+template <int N> __device__ __forceinline__ int warp_value(int lane) {
+  return N == 32 ? lane : lane >> 1;
+}
+
 // Deterministic grid reduction: every block writes its partials (nvals doubles) to
 // partials[block * nvals + k]; the block that arrives last (ticket) sees all of them.
 // Returns true in the last block (all threads), after which the caller sums the

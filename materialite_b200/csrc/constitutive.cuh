@@ -178,7 +178,9 @@ __device__ __forceinline__ void load6(const T *f, long long V, long long v, doub
 }
 
 // Threads of a constitutive block, and points of one item: four per thread, fewer (down to
-// one) where that many would leave the chip's blocks (three on each of 148 SMs) without one.
+// one) where that many would leave the chip's blocks (three on each of 148 SMs) without one.  V
+// counts the points of every listed slot: an item's results do not depend on its size (sixteen
+// slots of 32 x 8 x 256 float: 63 us a call sized for one, 38 so).
 #define CONST_THREADS 128
 #define CONST_ROUND_ITEMS 444
 
@@ -274,7 +276,7 @@ template <typename T>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     j2_count_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ int blk_n, blk_any, blk_fail;
-  const int chunk = const_chunk(V), per = const_items(V);
+  const int chunk = const_chunk(V * *list.count), per = (int)((V + chunk - 1) / chunk);
   const int n_items = list_items(list, per);
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
   const int kslot = item / per;
@@ -351,7 +353,7 @@ __global__ void __launch_bounds__(CONST_THREADS, 3)
 #define TS(arr, k) arr[(k) * CONST_THREADS]
   __shared__ int blk_max;
   __shared__ int blk_fail;
-  const int chunk = const_chunk(V), per = const_items(V);
+  const int chunk = const_chunk(V * *list.count), per = (int)((V + chunk - 1) / chunk);
   const int n_items = list_items(list, per);
   int staged = -1;  // slot whose phase table is in shared memory
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {

@@ -144,7 +144,7 @@ __device__ __forceinline__ double norm_combine(int k, double a, double b) {
   return k < NORM_SUMS ? a + b : fmax(a, b);
 }
 
-// Warp tree reduction of value k (fixed shuffle order).
+// Warp tree reduction of value k (fixed shuffle order; warp_reduce_many combines in it too).
 __device__ __forceinline__ double norm_warp_reduce(int k, double v) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) v = norm_combine(k, v, __shfl_down_sync(0xffffffffu, v, off));
@@ -154,57 +154,57 @@ __device__ __forceinline__ double norm_warp_reduce(int k, double v) {
 template <typename T>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     newton_norms_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
-  __shared__ double wred[NORM_VALS][SSFFT_THREADS / 32];
+  __shared__ double wred[VEC_GROUP_MAX][NORM_VALS][SSFFT_THREADS / 32];
   const int chunk = vec_chunk(V), per = vec_items(V);
-  const int n_items = list_items(list, per);
+  const ChunkGroups G = chunk_groups(list, per);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int kslot = item / per;
-    const int local = item - kslot * per;
+  for (int item = blockIdx.x; item < G.n_items; item += gridDim.x) {
+    const int kslot = item / G.groups;
+    const int first = (item - kslot * G.groups) * G.size, ng = min(G.size, per - first);
     const SlotDev<T> &S = tab[list.ids[kslot]];
     const T *dx = S.norms_dx ? S.kr[5] : nullptr;
     const TangentRef<T> K = tangent_of<T>(S, false, V);
-    double acc[NORM_VALS];
+    for (int j = 0; j < ng; ++j) {
+      double acc[16];
 #pragma unroll
-    for (int k = 0; k < NORM_VALS; ++k) acc[k] = 0.0;
-    const long long v0 = (long long)local * chunk;
-    const long long v1 = min(V, v0 + chunk);
-    for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
-      double s[6], d[6];
+      for (int k = 0; k < 16; ++k) acc[k] = 0.0;
+      const long long v0 = (long long)(first + j) * chunk;
+      const long long v1 = min(V, v0 + chunk);
+      for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+        double s[6], d[6];
 #pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        s[c] = (double)S.sig[c * V + v];
-        acc[c] += s[c];
-        acc[6 + c] += (double)S.eps[c * V + v];
-        d[c] = s[c] - (double)S.sig_old[c * V + v];
+        for (int c = 0; c < 6; ++c) {
+          s[c] = (double)S.sig[c * V + v];
+          acc[c] += s[c];
+          acc[6 + c] += (double)S.eps[c * V + v];
+          d[c] = s[c] - (double)S.sig_old[c * V + v];
+        }
+        acc[12] = fmax(acc[12], dev_norm6(d));
+        if (dx) {
+          double x[6], y[6];
+#pragma unroll
+          for (int c = 0; c < 6; ++c) x[c] = (double)dx[c * V + v];
+          K.apply(v, x, y);
+          double n2 = 0.0;
+#pragma unroll
+          for (int c = 0; c < 6; ++c) n2 += y[c] * y[c];
+          acc[13] = fmax(acc[13], sqrt(n2));
+        }
       }
-      acc[12] = fmax(acc[12], dev_norm6(d));
-      if (dx) {
-        double x[6], y[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) x[c] = (double)dx[c * V + v];
-        K.apply(v, x, y);
-        double n2 = 0.0;
-#pragma unroll
-        for (int c = 0; c < 6; ++c) n2 += y[c] * y[c];
-        acc[13] = fmax(acc[13], sqrt(n2));
+      // all fourteen values through one warp pass (70 shuffles as fourteen trees, 16 here)
+      const double r = warp_reduce_many<16>(acc, [](int k, double a, double b) { return norm_combine(k, a, b); });
+      const int k = warp_value<16>(lane);
+      if (k < NORM_VALS && (lane & 1) == 0) wred[j][k][warp] = r;
+    }
+    __syncthreads();
+    if (warp == 0)
+      for (int t = lane; t < ng * NORM_VALS; t += 32) {
+        const int j = t / NORM_VALS, k = t - j * NORM_VALS;
+        double r = wred[j][k][0];
+        for (int w = 1; w < nw; ++w) r = norm_combine(k, r, wred[j][k][w]);
+        S.partials[(size_t)first * NORM_VALS + t] = r;
       }
-    }
-    // all fourteen values through one warp pass and one barrier
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NORM_VALS; ++k) {
-      const double r = norm_warp_reduce(k, acc[k]);
-      if (lane == 0) wred[k][warp] = r;
-    }
-    __syncthreads();
-    if (threadIdx.x < NORM_VALS) {
-      const int k = threadIdx.x;
-      double r = wred[k][0];
-      for (int w = 1; w < nw; ++w) r = norm_combine(k, r, wred[k][w]);
-      S.partials[(size_t)local * NORM_VALS + k] = r;
-    }
-    if (last_item_arrives(S.tickets + TK_NORMS, (unsigned)per)) {
+    if (last_item_arrives(S.tickets + TK_NORMS, (unsigned)G.groups)) {
       // one warp per value: lanes stride over the item partials, then a fixed tree
       for (int k = warp; k < NORM_VALS; k += nw) {
         double r = 0.0;
@@ -225,28 +225,29 @@ template <typename T>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     tangent_sum_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ double red[32];
+  __shared__ double wsum[VEC_GROUP_MAX][21][8];
   const int chunk = vec_chunk(V), per = vec_items(V);
-  const int n_items = list_items(list, per);
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int kslot = item / per;
-    const int local = item - kslot * per;
+  const ChunkGroups G = chunk_groups(list, per);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int item = blockIdx.x; item < G.n_items; item += gridDim.x) {
+    const int kslot = item / G.groups;
+    const int first = (item - kslot * G.groups) * G.size, ng = min(G.size, per - first);
     const SlotDev<T> &S = tab[list.ids[kslot]];
     const TangentRef<T> K = tangent_of<T>(S, true, V);
-    double acc[21];
+    for (int j = 0; j < ng; ++j) {
+      double acc[32];
 #pragma unroll
-    for (int k = 0; k < 21; ++k) acc[k] = 0.0;
-    const long long v0 = (long long)local * chunk;
-    const long long v1 = min(V, v0 + chunk);
-    for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+      for (int k = 0; k < 32; ++k) acc[k] = 0.0;
+      const long long v0 = (long long)(first + j) * chunk;
+      const long long v1 = min(V, v0 + chunk);
+      for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
 #pragma unroll
-      for (int k = 0; k < 21; ++k) acc[k] += K.entry(v, k);
+        for (int k = 0; k < 21; ++k) acc[k] += K.entry(v, k);
+      }
+      const double r = warp_reduce_many<32>(acc, [](int, double a, double b) { return a + b; });
+      if (lane < 21) wsum[j][lane][warp] = r;
     }
-#pragma unroll
-    for (int k = 0; k < 21; ++k) {
-      const double r = block_sum(acc[k], red);
-      if (threadIdx.x == 0) S.partials[(size_t)local * 21 + k] = r;
-    }
-    if (last_item_arrives(S.tickets + TK_TSUM, (unsigned)per)) {
+    if (store_chunk_sums<21>(S.partials, S.tickets + TK_TSUM, G, first, ng, wsum)) {
       for (int k = 0; k < 21; ++k) {
         const double r = ordered_sum(S.partials + k, per, 21, red);
         if (threadIdx.x == 0) S.results[16 + k] = r;

@@ -34,8 +34,8 @@
 // SMs), at least one value a thread; above that 4096, so that the last round stays short.
 // With 4096 throughout, a 32^3 grid had 8 items on 148 SMs.  Measured, 4096 against this rule:
 // update 31.3 -> 13.8 us and epilogue 20.0 -> 12.3 us at 32^3 FP64, 26.8 -> 18.1 and 17.2 ->
-// 14.4 at 64^3 float, 97.9 -> 92.7 and 44.6 -> 40.5 at 128^3 float.  The size follows from the grid alone, never from the slots of a launch, so a slot's sums do not
-// depend on the batch.
+// 14.4 at 64^3 float, 97.9 -> 92.7 and 44.6 -> 40.5 at 128^3 float.  The size follows from the grid
+// alone, never from the slots of a launch, so a slot's sums do not depend on the batch.
 #define VEC_ROUND_ITEMS 296
 #define VEC_MAX_ROUND_CHUNK 8192
 #define VEC_LARGE_CHUNK 4096
@@ -50,35 +50,78 @@ __host__ __device__ inline int vec_items(long long n) {
   return (int)((n + c - 1) / c);
 }
 
+// Chunks of one slot that a block takes in a row where a launch has many slots: as many as leave
+// the grid one round, up to VEC_GROUP_MAX.  Each chunk keeps its own partial sum, formed from
+// its warps' sums in one fixed order, so the grouping (which follows the live slots) changes no
+// result; a group pays one pair of barriers, one fence and one ticket, and its warps run
+// ahead of one another.  Sixteen slots of 32 x 8 x 256 (256 chunks of 256 points each), us a
+// launch, chunk by chunk / in groups: update 94 / 56 float and 155 / 119 double, epilogue 98 / 27
+// and 88 / 39, norms 121 / 70 float.  With 4096 points a chunk, which starve a single slot, the
+// same launches take 51 and 105, 23 and 35, and 74.
+#define VEC_GROUP_MAX 8
+struct ChunkGroups {
+  int per, size, groups, n_items;  // chunks a slot, chunks a group, groups a slot, groups in all
+};
+__device__ __forceinline__ ChunkGroups chunk_groups(const SlotList &L, int per) {
+  const int count = *L.count;
+  ChunkGroups G;
+  G.per = per;
+  G.size = 1;
+  if (count > 1) {
+    const int m = max(1, (int)gridDim.x / count);
+    G.size = min(VEC_GROUP_MAX, (per + m - 1) / m);
+  }
+  G.groups = (per + G.size - 1) / G.size;
+  G.n_items = count * G.groups;
+  return G;
+}
+
+// Store the NV sums of a group's chunks first .. first + ng - 1 from the sums of the W warps that
+// took each; true in the block that completes the slot.
+template <int NV>
+__device__ __forceinline__ bool store_chunk_sums(double *partials, unsigned int *ticket,
+                                                 const ChunkGroups &G, int first, int ng,
+                                                 double (*wsum)[NV][8], int W = 8) {
+  __syncthreads();
+  if (threadIdx.x < 32)
+    for (int t = threadIdx.x; t < ng * NV; t += 32)
+      partials[(size_t)first * NV + t] = warps_sum(wsum[t / NV][t % NV], W);
+  return last_item_arrives(ticket, (unsigned)G.groups);
+}
+
 // Start of a solve on every listed slot: r1 = r2 = b, x = w = w2 = 0, |b|^2; the slot's
 // last item initialises its MINRES state.
 template <typename T>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     minres_init_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ double red[32];
+  __shared__ double wsum[VEC_GROUP_MAX][1][8];
   const long long n = 6 * V;
   const int chunk = vec_chunk(n), per = vec_items(n);
-  const int n_items = list_items(list, per);
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int k = item / per;
-    const int local = item - k * per;
+  const ChunkGroups G = chunk_groups(list, per);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int item = blockIdx.x; item < G.n_items; item += gridDim.x) {
+    const int k = item / G.groups;
+    const int first = (item - k * G.groups) * G.size, ng = min(G.size, per - first);
     const SlotDev<T> &S = tab[list.ids[k]];
     const KRoles<T> r = kroles<T>(S, 0);
-    const long long i0 = (long long)local * chunk;
-    const long long i1 = min(n, i0 + chunk);
-    double acc = 0.0;
-    for (long long i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-      const T bi = S.b[i];
-      r.P[i] = bi;
-      r.Q[i] = bi;
-      r.X[i] = 0;
-      r.W[i] = 0;
-      r.W2[i] = 0;
-      acc += (double)bi * (double)bi;
+    for (int j = 0; j < ng; ++j) {
+      const long long i0 = (long long)(first + j) * chunk;
+      const long long i1 = min(n, i0 + chunk);
+      double acc = 0.0;
+      for (long long i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+        const T bi = S.b[i];
+        r.P[i] = bi;
+        r.Q[i] = bi;
+        r.X[i] = 0;
+        r.W[i] = 0;
+        r.W2[i] = 0;
+        acc += (double)bi * (double)bi;
+      }
+      acc = warp_sum(acc);
+      if (lane == 0) wsum[j][0][warp] = acc;
     }
-    const double part = block_sum(acc, red);
-    if (threadIdx.x == 0) S.partials[local] = part;
-    if (last_item_arrives(S.tickets + TK_INIT, (unsigned)per)) {
+    if (store_chunk_sums<1>(S.partials, S.tickets + TK_INIT, G, first, ng, wsum)) {
       const double b2 = ordered_sum(S.partials, per, 1, red);
       if (threadIdx.x == 0) {
         S.tickets[TK_INIT] = 0;
@@ -140,34 +183,63 @@ template <typename T, int PRO>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     krylov_update_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ double red[32];
+  __shared__ double wsum[VEC_GROUP_MAX][1][8];
   __shared__ __align__(16) unsigned char sdesc[sizeof(SlotDev<T>)];
   const int chunk = vec_chunk(V), per = vec_items(V);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_begin();
   pdl_wait();
   const int slot0 = list.ids[blockIdx.x / per];  // read beside the count: a grid has no more blocks than the list can fill
-  const int n_items = list_items(list, per);
+  const ChunkGroups G = chunk_groups(list, per);
   int staged = -1;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int k = item / per;
-    const int local = item - k * per;
-    const int slot = item == (int)blockIdx.x ? slot0 : list.ids[k];
+  for (int item = blockIdx.x; item < G.n_items; item += gridDim.x) {
+    const int k = item / G.groups;
+    const int first = (item - k * G.groups) * G.size, ng = min(G.size, per - first);
+    const int slot = G.size == 1 && item == (int)blockIdx.x ? slot0 : list.ids[k];
     const MinresState *st = list.st + slot;
     const bool done = slot_done(st);
     KrylovIn<T, T> u = krylov_in<T, T>(st);
     const SlotDev<T> &S = stage_slot<T>(tab, slot, sdesc, staged);
     if (done) continue;
     u.r = kroles<T>(S, u.itn);
-    const long long v0 = (long long)local * chunk;
-    const long long v1 = min(V, v0 + chunk);
     T *tau_out = u.r.Y;
-    double xx = 0.0;
-    for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
-      T tau[6];
-      tangent_prologue<T, T, PRO, true>(S, V, v, u, 0, tau, xx);
+    for (int j = 0; j < ng; ++j) {
+      const long long v0 = (long long)(first + j) * chunk;
+      const long long v1 = min(V, v0 + chunk);
+      double xx = 0.0;
+      for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+        T tau[6];
+        tangent_prologue<T, T, PRO, true>(S, V, v, u, 0, tau, xx);
 #pragma unroll
-      for (int c = 0; c < 6; ++c) tau_out[c * V + v] = tau[c];
+        for (int c = 0; c < 6; ++c) tau_out[c * V + v] = tau[c];
+      }
+      xx = warp_sum(xx);
+      if (lane == 0) wsum[j][0][warp] = xx;
     }
-    if (u.on) finish_pending_update(S, xx, local, per, red);
+    // where a pending update was applied: the slot's |x|^2, then the stopping tests in its last
+    // group to arrive
+    if (u.on && store_chunk_sums<1>(S.partials, S.tickets + TK_UPD, G, first, ng, wsum)) {
+      const double x2 = ordered_sum(S.partials, per, 1, red);
+      if (threadIdx.x == 0) {
+        S.tickets[TK_UPD] = 0;
+        minres_after_update(S.st, x2);
+      }
+    }
+  }
+}
+
+// End of a group of the matvec epilogue: the three dot products, and in the slot's last group
+// the recurrence.
+template <typename T>
+__device__ __forceinline__ void finish_matvec(const SlotDev<T> &S, const ChunkGroups &G, int first, int ng,
+                                              double (*wsum)[3][8], int W, double *red) {
+  if (!store_chunk_sums<3>(S.partials, S.tickets + TK_ZINV, G, first, ng, wsum, W)) return;
+  const double d0 = ordered_sum(S.partials, G.per, 3, red);
+  const double d1 = ordered_sum(S.partials + 1, G.per, 3, red);
+  const double d2 = ordered_sum(S.partials + 2, G.per, 3, red);
+  if (threadIdx.x == 0) {
+    minres_after_matvec(S.st, d0, d1, d2);
+    S.tickets[TK_ZINV] = 0;
   }
 }
 
@@ -179,17 +251,19 @@ template <typename T>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     krylov_epilogue_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ double red[32];
+  __shared__ double wsum[VEC_GROUP_MAX][3][8];
   __shared__ __align__(16) unsigned char sdesc[sizeof(SlotDev<T>)];
   const int chunk = vec_chunk(V), per = vec_items(V);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_begin();
   pdl_wait();
   const int slot0 = list.ids[blockIdx.x / per];  // read beside the count: a grid has no more blocks than the list can fill
-  const int n_items = list_items(list, per);
+  const ChunkGroups G = chunk_groups(list, per);
   int staged = -1;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int k = item / per;
-    const int local = item - k * per;
-    const int slot = item == (int)blockIdx.x ? slot0 : list.ids[k];
+  for (int item = blockIdx.x; item < G.n_items; item += gridDim.x) {
+    const int k = item / G.groups;
+    const int first = (item - k * G.groups) * G.size, ng = min(G.size, per - first);
+    const int slot = G.size == 1 && item == (int)blockIdx.x ? slot0 : list.ids[k];
     const MinresState *st = list.st + slot;
     const bool done = slot_done(st);
     const long long itn = st->itn;
@@ -197,57 +271,82 @@ __global__ void __launch_bounds__(SSFFT_THREADS)
     const SlotDev<T> &S = stage_slot<T>(tab, slot, sdesc, staged);
     if (done) continue;
     const KRoles<T> kr = kroles<T>(S, itn);
-    const long long v0 = (long long)local * chunk;
-    const long long v1 = min(V, v0 + chunk);
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
     if constexpr (sizeof(T) == 4) {
       // four consecutive points a thread, one 16-byte load per component plane and vector
       // (each plane starts on a 16-byte boundary when V is a multiple of 4, and so does every
-      // item): four times the bytes in flight of one point a thread
+      // item): four times the bytes in flight of one point a thread.  A chunk of less than 1024
+      // points takes the first W warps' worth; a group's next chunks take the others
       if ((V & 3) == 0) {
-        for (long long v = v0 + 4 * threadIdx.x; v < v1; v += 4 * blockDim.x) {
-          float4 pt[6], r1[6], r2[6];
+        const int W = min(8, chunk >> 7), J = 8 / W, sub = warp / W, wl = warp - sub * W;
+        for (int j = sub; j < ng && sub < J; j += J) {
+          const long long v0 = (long long)(first + j) * chunk;
+          const long long v1 = min(V, v0 + chunk);
+          double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+          for (long long v = v0 + 4 * (32 * wl + lane); v < v1; v += 128 * W) {
+            float4 pt[6], r1[6], r2[6];
 #pragma unroll
-          for (int c = 0; c < 6; ++c) {
-            pt[c] = *reinterpret_cast<const float4 *>(kr.Y + c * V + v);
-            r1[c] = *reinterpret_cast<const float4 *>(kr.P + c * V + v);
-            r2[c] = *reinterpret_cast<const float4 *>(kr.Q + c * V + v);
+            for (int c = 0; c < 6; ++c) {
+              pt[c] = *reinterpret_cast<const float4 *>(kr.Y + c * V + v);
+              r1[c] = *reinterpret_cast<const float4 *>(kr.P + c * V + v);
+              r2[c] = *reinterpret_cast<const float4 *>(kr.Q + c * V + v);
+            }
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+              const float4 y = make_float4(pt[c].x - c1 * r1[c].x, pt[c].y - c1 * r1[c].y,
+                                           pt[c].z - c1 * r1[c].z, pt[c].w - c1 * r1[c].w);
+              *reinterpret_cast<float4 *>(kr.Y + c * V + v) = y;
+              a0 += (double)r2[c].x * (double)y.x + (double)r2[c].y * (double)y.y +
+                    (double)r2[c].z * (double)y.z + (double)r2[c].w * (double)y.w;
+              a1 += (double)y.x * (double)y.x + (double)y.y * (double)y.y +
+                    (double)y.z * (double)y.z + (double)y.w * (double)y.w;
+              a2 += (double)r2[c].x * (double)r2[c].x + (double)r2[c].y * (double)r2[c].y +
+                    (double)r2[c].z * (double)r2[c].z + (double)r2[c].w * (double)r2[c].w;
+            }
           }
-#pragma unroll
-          for (int c = 0; c < 6; ++c) {
-            const float4 y = make_float4(pt[c].x - c1 * r1[c].x, pt[c].y - c1 * r1[c].y,
-                                         pt[c].z - c1 * r1[c].z, pt[c].w - c1 * r1[c].w);
-            *reinterpret_cast<float4 *>(kr.Y + c * V + v) = y;
-            a0 += (double)r2[c].x * (double)y.x + (double)r2[c].y * (double)y.y +
-                  (double)r2[c].z * (double)y.z + (double)r2[c].w * (double)y.w;
-            a1 += (double)y.x * (double)y.x + (double)y.y * (double)y.y +
-                  (double)y.z * (double)y.z + (double)y.w * (double)y.w;
-            a2 += (double)r2[c].x * (double)r2[c].x + (double)r2[c].y * (double)r2[c].y +
-                  (double)r2[c].z * (double)r2[c].z + (double)r2[c].w * (double)r2[c].w;
+          a0 = warp_sum(a0);
+          a1 = warp_sum(a1);
+          a2 = warp_sum(a2);
+          if (lane == 0) {
+            wsum[j][0][wl] = a0;
+            wsum[j][1][wl] = a1;
+            wsum[j][2][wl] = a2;
           }
         }
-        finish_inverse<T, EPI_MINRES>(S, a0, a1, a2, local, per, red);
+        finish_matvec(S, G, first, ng, wsum, W, red);
         continue;
       }
     }
-    for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
-      T pt[6], r1[6], r2[6];
+    for (int j = 0; j < ng; ++j) {
+      const long long v0 = (long long)(first + j) * chunk;
+      const long long v1 = min(V, v0 + chunk);
+      double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+      for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+        T pt[6], r1[6], r2[6];
 #pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        pt[c] = kr.Y[c * V + v];
-        r1[c] = kr.P[c * V + v];
-        r2[c] = kr.Q[c * V + v];
+        for (int c = 0; c < 6; ++c) {
+          pt[c] = kr.Y[c * V + v];
+          r1[c] = kr.P[c * V + v];
+          r2[c] = kr.Q[c * V + v];
+        }
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+          const T y = pt[c] - c1 * r1[c];
+          kr.Y[c * V + v] = y;
+          a0 += (double)r2[c] * (double)y;
+          a1 += (double)y * (double)y;
+          a2 += (double)r2[c] * (double)r2[c];
+        }
       }
-#pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        const T y = pt[c] - c1 * r1[c];
-        kr.Y[c * V + v] = y;
-        a0 += (double)r2[c] * (double)y;
-        a1 += (double)y * (double)y;
-        a2 += (double)r2[c] * (double)r2[c];
+      a0 = warp_sum(a0);
+      a1 = warp_sum(a1);
+      a2 = warp_sum(a2);
+      if (lane == 0) {
+        wsum[j][0][warp] = a0;
+        wsum[j][1][warp] = a1;
+        wsum[j][2][warp] = a2;
       }
     }
-    finish_inverse<T, EPI_MINRES>(S, a0, a1, a2, local, per, red);
+    finish_matvec(S, G, first, ng, wsum, 8, red);
   }
 }
 

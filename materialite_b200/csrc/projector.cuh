@@ -374,21 +374,6 @@ __device__ __forceinline__ void tangent_prologue(const SlotDev<TF> &S, long long
   }
 }
 
-// End of a forward item that applied a pending update: the slot's |x|^2 over its items,
-// then the stopping tests in the slot's last item to arrive.
-template <typename TF>
-__device__ __forceinline__ void finish_pending_update(const SlotDev<TF> &S, double xx, int local,
-                                                      int per_slot, double *red) {
-  const double part = block_sum(xx, red);
-  if (threadIdx.x == 0) S.partials[local] = part;
-  if (!last_item_arrives(S.tickets + TK_UPD, (unsigned)per_slot)) return;
-  const double x2 = ordered_sum(S.partials, per_slot, 1, red);
-  if (threadIdx.x == 0) {
-    S.tickets[TK_UPD] = 0;
-    minres_after_update(S.st, x2);
-  }
-}
-
 template <typename T>
 __device__ __forceinline__ void load_table(cplx<T> *dst, const cplx<T> *src, int n) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
@@ -426,8 +411,7 @@ __device__ __forceinline__ void epilogue_point(const SlotDev<TF> &S, const ExtIO
   }
 }
 
-// End of an inverse item: the slot's max |b| (residual) or its three MINRES dot products,
-// finished by the slot's last item.
+// End of an inverse item: the slot's max |b| (residual), finished by the slot's last item.
 template <typename TF, int EPI>
 __device__ __forceinline__ void finish_inverse(const SlotDev<TF> &S, double acc0, double acc1,
                                                double acc2, int local, int per_slot,
@@ -435,31 +419,10 @@ __device__ __forceinline__ void finish_inverse(const SlotDev<TF> &S, double acc0
   if constexpr (EPI == EPI_RESIDUAL) {
     const double part = block_max(acc0, red);
     if (threadIdx.x == 0) S.partials[local] = part;
-  } else if constexpr (EPI == EPI_MINRES) {
-    const double q0 = block_sum(acc0, red);
-    const double q1 = block_sum(acc1, red);
-    const double q2 = block_sum(acc2, red);
-    if (threadIdx.x == 0) {
-      S.partials[3 * local] = q0;
-      S.partials[3 * local + 1] = q1;
-      S.partials[3 * local + 2] = q2;
-    }
-  } else {
-    return;
-  }
-  if (!last_item_arrives(S.tickets + TK_ZINV, (unsigned)per_slot)) return;
-  if constexpr (EPI == EPI_RESIDUAL) {
+    if (!last_item_arrives(S.tickets + TK_ZINV, (unsigned)per_slot)) return;
     const double m = ordered_max(S.partials, per_slot, 1, red);
     if (threadIdx.x == 0) {
       S.results[40] = m;
-      S.tickets[TK_ZINV] = 0;
-    }
-  } else {
-    const double d0 = ordered_sum(S.partials, per_slot, 3, red);
-    const double d1 = ordered_sum(S.partials + 1, per_slot, 3, red);
-    const double d2 = ordered_sum(S.partials + 2, per_slot, 3, red);
-    if (threadIdx.x == 0) {
-      minres_after_matvec(S.st, d0, d1, d2);
       S.tickets[TK_ZINV] = 0;
     }
   }
