@@ -274,9 +274,9 @@ __device__ __forceinline__ double j2_update(const PhaseParams &P, double q, doub
 // J2_MAX_ITERATIONS fails the update (:133-137).
 template <typename T>
 __global__ void __launch_bounds__(SSFFT_THREADS)
-    j2_count_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
+    j2_count_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V, int many) {
   __shared__ int blk_n, blk_any, blk_fail;
-  const int chunk = const_chunk(V * *list.count), per = (int)((V + chunk - 1) / chunk);
+  const int chunk = const_chunk(many ? V * *list.count : V), per = (int)((V + chunk - 1) / chunk);
   const int n_items = list_items(list, per);
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
   const int kslot = item / per;
@@ -340,7 +340,7 @@ inline size_t constitutive_smem_bytes() {
 
 template <typename T>
 __global__ void __launch_bounds__(CONST_THREADS, 3)
-    constitutive_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
+    constitutive_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V, int many) {
   extern __shared__ __align__(16) unsigned char csm[];
   PhaseParams *sp = reinterpret_cast<PhaseParams *>(csm);
   const int tid = threadIdx.x;
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(CONST_THREADS, 3)
 #define TS(arr, k) arr[(k) * CONST_THREADS]
   __shared__ int blk_max;
   __shared__ int blk_fail;
-  const int chunk = const_chunk(V * *list.count), per = (int)((V + chunk - 1) / chunk);
+  const int chunk = const_chunk(many ? V * *list.count : V), per = (int)((V + chunk - 1) / chunk);
   const int n_items = list_items(list, per);
   int staged = -1;  // slot whose phase table is in shared memory
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {

@@ -151,16 +151,16 @@ __device__ __forceinline__ double norm_warp_reduce(int k, double v) {
   return v;
 }
 
-template <typename T>
+template <typename T, bool MANY>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     newton_norms_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
-  __shared__ double wred[VEC_GROUP_MAX][NORM_VALS][SSFFT_THREADS / 32];
+  __shared__ double wred[MANY ? VEC_GROUP_MAX : 1][NORM_VALS][SSFFT_THREADS / 32];
   const int chunk = vec_chunk(V), per = vec_items(V);
-  const ChunkGroups G = chunk_groups(list, per);
+  const ChunkGroups G = chunk_groups<MANY>(list, per);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int item = blockIdx.x; item < G.n_items; item += gridDim.x) {
     const int kslot = item / G.groups;
-    const int first = (item - kslot * G.groups) * G.size, ng = min(G.size, per - first);
+    const int first = (item - kslot * G.groups) * G.size, ng = MANY ? min(G.size, per - first) : 1;
     const SlotDev<T> &S = tab[list.ids[kslot]];
     const T *dx = S.norms_dx ? S.kr[5] : nullptr;
     const TangentRef<T> K = tangent_of<T>(S, false, V);
@@ -221,17 +221,17 @@ __global__ void __launch_bounds__(SSFFT_THREADS)
 
 // Sum of the committed tangent over all points (21 packed entries) for
 // tangent.mean().inv (small_strain_fft.py:119-120), into results[16..36].
-template <typename T>
+template <typename T, bool MANY>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     tangent_sum_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ double red[32];
-  __shared__ double wsum[VEC_GROUP_MAX][21][8];
+  __shared__ double wsum[MANY ? VEC_GROUP_MAX : 1][21][8];
   const int chunk = vec_chunk(V), per = vec_items(V);
-  const ChunkGroups G = chunk_groups(list, per);
+  const ChunkGroups G = chunk_groups<MANY>(list, per);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int item = blockIdx.x; item < G.n_items; item += gridDim.x) {
     const int kslot = item / G.groups;
-    const int first = (item - kslot * G.groups) * G.size, ng = min(G.size, per - first);
+    const int first = (item - kslot * G.groups) * G.size, ng = MANY ? min(G.size, per - first) : 1;
     const SlotDev<T> &S = tab[list.ids[kslot]];
     const TangentRef<T> K = tangent_of<T>(S, true, V);
     for (int j = 0; j < ng; ++j) {

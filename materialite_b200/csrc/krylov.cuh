@@ -62,16 +62,20 @@ __host__ __device__ inline int vec_items(long long n) {
 struct ChunkGroups {
   int per, size, groups, n_items;  // chunks a slot, chunks a group, groups a slot, groups in all
 };
-__device__ __forceinline__ ChunkGroups chunk_groups(const SlotList &L, int per) {
+// MANY: the list can hold more than one slot.  A handle's kernels are compiled without groups:
+// with them the FP64 update took 1 to 3 us more a launch (64^3 31.8 and 33.1 us, 128^3 181.6
+// and 184.6).
+template <bool MANY> __device__ __forceinline__ ChunkGroups chunk_groups(const SlotList &L, int per) {
   const int count = *L.count;
   ChunkGroups G;
   G.per = per;
   G.size = 1;
-  if (count > 1) {
+  G.groups = per;
+  if (MANY && count > 1) {
     const int m = max(1, (int)gridDim.x / count);
     G.size = min(VEC_GROUP_MAX, (per + m - 1) / m);
+    G.groups = (per + G.size - 1) / G.size;
   }
-  G.groups = (per + G.size - 1) / G.size;
   G.n_items = count * G.groups;
   return G;
 }
@@ -91,18 +95,18 @@ __device__ __forceinline__ bool store_chunk_sums(double *partials, unsigned int 
 
 // Start of a solve on every listed slot: r1 = r2 = b, x = w = w2 = 0, |b|^2; the slot's
 // last item initialises its MINRES state.
-template <typename T>
+template <typename T, bool MANY>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     minres_init_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ double red[32];
-  __shared__ double wsum[VEC_GROUP_MAX][1][8];
+  __shared__ double wsum[MANY ? VEC_GROUP_MAX : 1][1][8];
   const long long n = 6 * V;
   const int chunk = vec_chunk(n), per = vec_items(n);
-  const ChunkGroups G = chunk_groups(list, per);
+  const ChunkGroups G = chunk_groups<MANY>(list, per);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int item = blockIdx.x; item < G.n_items; item += gridDim.x) {
     const int k = item / G.groups;
-    const int first = (item - k * G.groups) * G.size, ng = min(G.size, per - first);
+    const int first = (item - k * G.groups) * G.size, ng = MANY ? min(G.size, per - first) : 1;
     const SlotDev<T> &S = tab[list.ids[k]];
     const KRoles<T> r = kroles<T>(S, 0);
     for (int j = 0; j < ng; ++j) {
@@ -179,23 +183,23 @@ __global__ void __launch_bounds__(SSFFT_THREADS)
 // iteration writes the next y' there).  The forward transform then copies tau from there
 // (PRO_TAU).  A plain streaming kernel: each point's loads go out together and no register
 // cap is imposed, so the loads of a block keep HBM busy.
-template <typename T, int PRO>
+template <typename T, int PRO, bool MANY>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     krylov_update_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ double red[32];
-  __shared__ double wsum[VEC_GROUP_MAX][1][8];
+  __shared__ double wsum[MANY ? VEC_GROUP_MAX : 1][1][8];
   __shared__ __align__(16) unsigned char sdesc[sizeof(SlotDev<T>)];
   const int chunk = vec_chunk(V), per = vec_items(V);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_begin();
   pdl_wait();
   const int slot0 = list.ids[blockIdx.x / per];  // read beside the count: a grid has no more blocks than the list can fill
-  const ChunkGroups G = chunk_groups(list, per);
+  const ChunkGroups G = chunk_groups<MANY>(list, per);
   int staged = -1;
   for (int item = blockIdx.x; item < G.n_items; item += gridDim.x) {
     const int k = item / G.groups;
-    const int first = (item - k * G.groups) * G.size, ng = min(G.size, per - first);
-    const int slot = G.size == 1 && item == (int)blockIdx.x ? slot0 : list.ids[k];
+    const int first = (item - k * G.groups) * G.size, ng = MANY ? min(G.size, per - first) : 1;
+    const int slot = (!MANY || G.size == 1) && item == (int)blockIdx.x ? slot0 : list.ids[k];
     const MinresState *st = list.st + slot;
     const bool done = slot_done(st);
     KrylovIn<T, T> u = krylov_in<T, T>(st);
@@ -247,23 +251,23 @@ __device__ __forceinline__ void finish_matvec(const SlotDev<T> &S, const ChunkGr
 // transform left in y''s buffer (EPI_PTAU), y' = P tau - (beta_j / beta_{j-1}) u_{j-1} in
 // place, and the dot products u_j.y', y'.y', u_j.u_j; the slot's last item advances the
 // recurrence (minres_after_matvec).
-template <typename T>
+template <typename T, bool MANY>
 __global__ void __launch_bounds__(SSFFT_THREADS)
     krylov_epilogue_kernel(const SlotDev<T> *__restrict__ tab, SlotList list, long long V) {
   __shared__ double red[32];
-  __shared__ double wsum[VEC_GROUP_MAX][3][8];
+  __shared__ double wsum[MANY ? VEC_GROUP_MAX : 1][3][8];
   __shared__ __align__(16) unsigned char sdesc[sizeof(SlotDev<T>)];
   const int chunk = vec_chunk(V), per = vec_items(V);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_begin();
   pdl_wait();
   const int slot0 = list.ids[blockIdx.x / per];  // read beside the count: a grid has no more blocks than the list can fill
-  const ChunkGroups G = chunk_groups(list, per);
+  const ChunkGroups G = chunk_groups<MANY>(list, per);
   int staged = -1;
   for (int item = blockIdx.x; item < G.n_items; item += gridDim.x) {
     const int k = item / G.groups;
-    const int first = (item - k * G.groups) * G.size, ng = min(G.size, per - first);
-    const int slot = G.size == 1 && item == (int)blockIdx.x ? slot0 : list.ids[k];
+    const int first = (item - k * G.groups) * G.size, ng = MANY ? min(G.size, per - first) : 1;
+    const int slot = (!MANY || G.size == 1) && item == (int)blockIdx.x ? slot0 : list.ids[k];
     const MinresState *st = list.st + slot;
     const bool done = slot_done(st);
     const long long itn = st->itn;

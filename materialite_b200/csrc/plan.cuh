@@ -1251,18 +1251,19 @@ static int launch_krylov_iteration(const LaunchCtx &c, const SlotDev<T> *tab, bo
                                    cudaEvent_t *ev = nullptr, bool pdl_first = false) {
   if (ev) cudaEventRecord(ev[7], c.stream);
   const long long it = (long long)c.cap * vec_items(c.p->V);
+  const bool many = c.cap > 1;
   if (voxel) {
-    auto k = krylov_update_kernel<T, PRO_TANGENT_VOXEL>;
+    auto k = many ? krylov_update_kernel<T, PRO_TANGENT_VOXEL, true> : krylov_update_kernel<T, PRO_TANGENT_VOXEL, false>;
     CKR(launch_kernel(pdl_first, k, persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0,
                       c.stream, tab, c.list, c.p->V));
   } else {
-    auto k = krylov_update_kernel<T, PRO_TANGENT_TABLE>;
+    auto k = many ? krylov_update_kernel<T, PRO_TANGENT_TABLE, true> : krylov_update_kernel<T, PRO_TANGENT_TABLE, false>;
     CKR(launch_kernel(pdl_first, k, persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0,
                       c.stream, tab, c.list, c.p->V));
   }
   if (c.launches) *c.launches += 1;
   CKR((launch_projector<T, T, PRO_TAU, EPI_PTAU>(c, tab, {}, ev)));
-  auto ke = krylov_epilogue_kernel<T>;
+  auto ke = many ? krylov_epilogue_kernel<T, true> : krylov_epilogue_kernel<T, false>;
   CKR(launch_kernel(true, ke, persistent_grid(ke, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0,
                     c.stream, tab, c.list, c.p->V));
   if (c.launches) *c.launches += 1;
@@ -1289,7 +1290,7 @@ template <typename T> static int launch_reproject_update(const LaunchCtx &c, con
 
 template <typename T>
 static int launch_minres_init(const LaunchCtx &c, const SlotDev<T> *tab) {
-  auto k = minres_init_kernel<T>;
+  auto k = c.cap > 1 ? minres_init_kernel<T, true> : minres_init_kernel<T, false>;
   const long long it = (long long)c.cap * vec_items(6 * c.p->V);
   k<<<persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0, c.stream>>>(tab, c.list, c.p->V);
   if (c.launches) *c.launches += 1;
@@ -1316,7 +1317,7 @@ template <typename T> static int launch_update_strain(const LaunchCtx &c, const 
 }
 
 template <typename T> static int launch_norms(const LaunchCtx &c, const SlotDev<T> *tab) {
-  auto k = newton_norms_kernel<T>;
+  auto k = c.cap > 1 ? newton_norms_kernel<T, true> : newton_norms_kernel<T, false>;
   const long long it = (long long)c.cap * vec_items(c.p->V);
   k<<<persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0, c.stream>>>(tab, c.list, c.p->V);
   if (c.launches) *c.launches += 1;
@@ -1325,7 +1326,7 @@ template <typename T> static int launch_norms(const LaunchCtx &c, const SlotDev<
 }
 
 template <typename T> static int launch_tangent_sum(const LaunchCtx &c, const SlotDev<T> *tab) {
-  auto k = tangent_sum_kernel<T>;
+  auto k = c.cap > 1 ? tangent_sum_kernel<T, true> : tangent_sum_kernel<T, false>;
   const long long it = (long long)c.cap * vec_items(c.p->V);
   k<<<persistent_grid(k, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0, c.stream>>>(tab, c.list, c.p->V);
   if (c.launches) *c.launches += 1;
@@ -1340,13 +1341,14 @@ static int launch_constitutive(const LaunchCtx &c, const SlotDev<T> *tab, bool j
   const long long it = (long long)c.cap * const_items(c.p->V);
   if (j2) {
     auto kj = j2_count_kernel<T>;
-    kj<<<persistent_grid(kj, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0, c.stream>>>(tab, c.list, c.p->V);
+    kj<<<persistent_grid(kj, SSFFT_THREADS, 0, it, c.p->dev), SSFFT_THREADS, 0, c.stream>>>(tab, c.list, c.p->V,
+                                                                                            c.cap > 1);
     if (c.launches) *c.launches += 1;
     CK(cudaGetLastError());
   }
   const size_t sm = constitutive_smem_bytes();
   auto k = constitutive_kernel<T>;
-  k<<<persistent_grid(k, CONST_THREADS, sm, it, c.p->dev), CONST_THREADS, sm, c.stream>>>(tab, c.list, c.p->V);
+  k<<<persistent_grid(k, CONST_THREADS, sm, it, c.p->dev), CONST_THREADS, sm, c.stream>>>(tab, c.list, c.p->V, c.cap > 1);
   if (c.launches) *c.launches += 1;
   CK(cudaGetLastError());
   return 0;
